@@ -308,9 +308,8 @@ int attn_step(const AttnDev &A, StateDev &S, const float *x, long long pos, cons
     return qlinear_dev(A.wo_b, b.y, out, B, b.xq, b.xs, true, st);
 }
 
-// The compressor over a chunk: the two projections of every row at once, then the state machine
-// position by position (it is sequential in t by definition, c/attn.h:960-1008; a launch per
-// position on B CTAs) with the entries it completes appended as it goes.
+// The compressor over a chunk: the two projections of every row at once, the entries the chunk completes
+// pooled together (comp_chunk), then finished and appended as rows of one launch.
 static int compressor_chunk(const CompDev &W, CompStateDev &S, const float *x, int B, int s, int dim, long long pos0,
                             const float *cs_table, const StepBufs &b0, cudaStream_t st, bool second_set = false) {
     StepBufs b = b0;
@@ -318,20 +317,17 @@ static int compressor_chunk(const CompDev &W, CompStateDev &S, const float *x, i
     const int cd = (1 + W.overlap) * W.d, T = B * s;
     if (comp_project(W, x, b.ckv, b.csc, T, dim, cd, st)) return 1;
     const int flags = ROW_BF16_IN | ROW_RMS_W | ROW_ROPE | ROW_BF16_OUT | (W.rotate ? (ROW_HADAMARD | ROW_FP4QAT) : ROW_FP8QAT);
-    for (int t = 0; t < s; t++) {
-        const long long pos = pos0 + t;
-        const int slot = (int)(pos % W.ratio), should = (pos + 1) % W.ratio == 0;
-        float *pooled = b.pooled + (size_t)t * B * W.d;
-        if (comp_step(S.kv.as<float>(), S.sc.as<float>(), (long long)S.carry, b.ckv + (size_t)t * B * cd,
-                      b.csc + (size_t)t * B * cd, cd, W.ape, W.ratio, W.overlap, W.d, slot, should, pooled, W.d, B, st))
-            return 1;
-        if (!should) continue;
-        APUS_REQUIRE(S.nb < S.cap, "compressed cache is full (%d entries)", S.cap);
-        if (row_ops(pooled, W.d, S.cache.as<float>() + (size_t)S.nb * W.d, S.cap * W.d, B, W.d, flags, W.norm, W.eps,
-                    W.rd, cs_table + (size_t)(pos + 1 - W.ratio) * W.rd, B, 0, st))
-            return 1;
-        S.nb++;
-    }
+    const int done = (int)((pos0 + s) / W.ratio - pos0 / W.ratio);
+    APUS_REQUIRE(S.nb + done <= S.cap, "compressed cache is full (%d entries)", S.cap);
+    if (comp_chunk(S.kv.as<float>(), S.sc.as<float>(), (long long)S.carry, b.ckv, b.csc, W.ape, W.ratio, W.overlap, W.d, pos0,
+                   s, B, b.pooled, st))
+        return 1;
+    // entry e of sequence q: row e * B + q, rotated by the first position of its block, appended at S.nb + e
+    if (row_ops(b.pooled, W.d, S.cache.as<float>() + (size_t)S.nb * W.d, S.cap * W.d, done * B, W.d, flags, W.norm, W.eps,
+                W.rd, cs_table + (size_t)(pos0 / W.ratio) * W.ratio * W.rd, B, W.ratio * W.rd, st, nullptr, nullptr, nullptr, B,
+                W.d))
+        return 1;
+    S.nb += done;
     return 0;
 }
 

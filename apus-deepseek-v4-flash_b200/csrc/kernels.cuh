@@ -232,13 +232,21 @@ struct RowDyn {
 };
 int row_ops(const float *x, int x_stride, float *y, int y_stride, int rows, int n, int flags,
             const float *norm_w, float eps, int rd, const float *cs, int rows_per_cs, int cs_stride,
-            cudaStream_t st, const RowDyn *dyn = nullptr, uint8_t *q_codes = nullptr, float *q_scales = nullptr);
+            cudaStream_t st, const RowDyn *dyn = nullptr, uint8_t *q_codes = nullptr, float *q_scales = nullptr,
+            int y_inner = 0, long long y_outer = 0);
+// y_inner > 0: output row r goes to y + (r / y_inner) * y_outer + (r % y_inner) * y_stride.
 // q_codes != NULL (n % 128 == 0): the finished rows are also written as the E4M3 codes [rows, n] and the
 // per-128 scales [rows, n / 128] that act_quant would make of y -- the same arithmetic, one launch less.
 int comp_step(float *kv_state, float *sc_state, long long state_stride, const float *kv_new,
               const float *sc_new, int new_stride, const float *ape, int ratio, int overlap, int d,
               int slot, int should, float *pooled, int pooled_stride, int n_seq, cudaStream_t st,
               const long long *dyn_pos = nullptr);    // dyn_pos: slot and should derived from *dyn_pos
+// The same over s consecutive positions from pos0, rows kv_new / sc_new time-major (t * n_seq + seq, width cd):
+// entry e of the (pos0 + s) / ratio - pos0 / ratio that complete is pooled into row e * n_seq + seq of
+// `pooled` (width d), the state is left as after the last position.
+int comp_chunk(float *kv_state, float *sc_state, long long state_stride, const float *kv_new, const float *sc_new,
+               const float *ape, int ratio, int overlap, int d, long long pos0, int s, int n_seq, float *pooled,
+               cudaStream_t st);
 // n_seq sequences in lockstep: q [n_seq, ih*idm], wt_raw [n_seq, ih], caches cache_stride floats
 // apart, sc [n_seq, nb].
 int idx_scores(const float *q, const float *wt_raw, float wscale, const float *cache, long long cache_stride,

@@ -64,6 +64,56 @@ mhc_mix_kernel(const float *__restrict__ x4, const float *__restrict__ fn, int n
     if (threadIdx.x == 0) raw[(size_t)row * (nmix + 1) + j] = tot;
 }
 
+// The same sums for many rows: TOK rows and JT of the nmix + 1 dots per CTA, so that a word of fn is read from
+// L2 once per TOK rows and a word of the state once per JT dots (the kernel above reads both once per dot and
+// row: bound by L2).  A thread adds the same terms in the same order as there, and so do the two shuffle stages
+// of the block sum: the same bits.  B200, 2,048 rows of 4 x 4096: 339 -> 149 us.
+template <int TOK, int JT>
+__global__ void __launch_bounds__(256)
+mhc_mix_rows_kernel(const float *__restrict__ x4, const float *__restrict__ fn, int nx, int nmix, int rows,
+                    float *__restrict__ raw) {
+    APUS_PDL_WAIT();
+    APUS_PDL_GO();
+    __shared__ float red[TOK * JT][8];
+    const int j0 = blockIdx.x * JT, row0 = blockIdx.y * TOK, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float acc[JT][TOK];
+#pragma unroll
+    for (int j = 0; j < JT; j++)
+#pragma unroll
+        for (int t = 0; t < TOK; t++) acc[j][t] = 0.f;
+    for (int i = tid * 4; i < nx; i += 1024) {
+        float4 b[TOK];
+#pragma unroll
+        for (int t = 0; t < TOK; t++)
+            b[t] = row0 + t < rows ? *reinterpret_cast<const float4 *>(x4 + (size_t)(row0 + t) * nx + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < JT; j++) {
+            const bool sq = j0 + j == nmix;              // the last chain is the sum of squares
+            float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (j0 + j < nmix) f = __ldg(reinterpret_cast<const float4 *>(fn + (size_t)(j0 + j) * nx + i));
+#pragma unroll
+            for (int t = 0; t < TOK; t++) {
+                const float4 a = sq ? b[t] : f;
+                acc[j][t] = fmaf(a.x, b[t].x, acc[j][t]); acc[j][t] = fmaf(a.y, b[t].y, acc[j][t]);
+                acc[j][t] = fmaf(a.z, b[t].z, acc[j][t]); acc[j][t] = fmaf(a.w, b[t].w, acc[j][t]);
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < JT; j++)
+#pragma unroll
+        for (int t = 0; t < TOK; t++) {
+            const float v = warp_sum(acc[j][t]);
+            if (lane == 0) red[j * TOK + t][warp] = v;
+        }
+    __syncthreads();
+    for (int o = warp; o < TOK * JT; o += 8) {
+        const float v = warp_sum(lane < 8 ? red[o][lane] : 0.f);
+        const int j = j0 + o / TOK, r = row0 + o % TOK;
+        if (lane == 0 && j <= nmix && r < rows) raw[(size_t)r * (nmix + 1) + j] = v;
+    }
+}
+
 // The same dots in the reference's summation order (c/mhc.h:159-176: one f32
 // accumulator per dot, products rounded before each add, index ascending).
 // That order is a chain of n*d dependent adds per dot, so the kernel is bound
@@ -471,8 +521,113 @@ mhc_pre_finish_cl_kernel(const float *__restrict__ x4, const float *__restrict__
         mhc_gates_warp(rw, r, n, scale, base, hc_eps, iters, (size_t)row, post_out, comb_out, tid);
 }
 
+// The same step for many rows, reference order of the norm's sum: one CTA per row.  With rows enough to fill the
+// GPU the cluster above only divides the shared memory a row needs over eight SMs and adds three cluster
+// barriers; here eight rows share an SM and one row's chain of d adds hides behind the others' loads.  A thread
+// keeps its R words of the collapsed row in registers between the two halves.  B200, 2,048 rows of 4 x 4096: 235 -> 72 us.
+template <int R>
+__global__ void __launch_bounds__(256)
+mhc_pre_finish_rows_kernel(const float *__restrict__ x4, const float *__restrict__ raw, int d, int n, int nmix,
+                           const float *__restrict__ scale, float head_scale, const float *__restrict__ base, float norm_eps,
+                           float hc_eps, int iters, int head_mode, const float *__restrict__ norm_w, float rms_eps,
+                           float *__restrict__ pre_out, float *__restrict__ post_out, float *__restrict__ comb_out,
+                           float *__restrict__ y, float *__restrict__ y_normed) {
+    APUS_PDL_WAIT();
+    APUS_PDL_GO();
+    extern __shared__ __align__(16) float s_sq[];   // the d squares of the collapsed row
+    __shared__ float s_pre[MHC_MAX_N];
+    __shared__ float s_tot;
+    const int row = blockIdx.x, tid = threadIdx.x;
+    const float *rw = raw + (size_t)row * (nmix + 1);
+    const float mean = __fdiv_rn(rw[nmix], (float)(n * d));
+    const float r = __fdiv_rn(1.0f, sqrtf(__fadd_rn(mean, norm_eps)));
+    if (tid < n) {
+        const float m = __fmul_rn(rw[tid], r);
+        const float sc = head_mode ? head_scale : scale[0];
+        s_pre[tid] = __fadd_rn(sigm(__fadd_rn(__fmul_rn(m, sc), base[tid])), hc_eps);
+        if (pre_out) pre_out[(size_t)row * n + tid] = s_pre[tid];
+    }
+    __syncthreads();
+    const float *x = x4 + (size_t)row * n * d;
+    float4 acc[R];
+#pragma unroll
+    for (int u = 0; u < R; u++) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < n; j++) {
+        const float p = s_pre[j];
+#pragma unroll
+        for (int u = 0; u < R; u++) {
+            const int i = 4 * (tid + 256 * u);
+            if (i >= d) continue;
+            const float4 v = *reinterpret_cast<const float4 *>(x + (size_t)j * d + i);
+            acc[u].x = __fadd_rn(acc[u].x, __fmul_rn(p, v.x)); acc[u].y = __fadd_rn(acc[u].y, __fmul_rn(p, v.y));
+            acc[u].z = __fadd_rn(acc[u].z, __fmul_rn(p, v.z)); acc[u].w = __fadd_rn(acc[u].w, __fmul_rn(p, v.w));
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+        const int i = 4 * (tid + 256 * u);
+        if (i >= d) continue;
+        acc[u].x = bf16_round(acc[u].x); acc[u].y = bf16_round(acc[u].y);
+        acc[u].z = bf16_round(acc[u].z); acc[u].w = bf16_round(acc[u].w);
+        *reinterpret_cast<float4 *>(y + (size_t)row * d + i) = acc[u];
+        *reinterpret_cast<float4 *>(s_sq + i) = make_float4(__fmul_rn(acc[u].x, acc[u].x), __fmul_rn(acc[u].y, acc[u].y),
+                                                            __fmul_rn(acc[u].z, acc[u].z), __fmul_rn(acc[u].w, acc[u].w));
+    }
+    __syncthreads();
+    if (tid == 0 && y_normed) s_tot = seq_sum_smem(s_sq, d, 0.f);
+    if ((tid >> 5) == 1 && !head_mode) mhc_gates_warp(rw, r, n, scale, base, hc_eps, iters, (size_t)row, post_out, comb_out, tid);
+    if (!y_normed) return;
+    __syncthreads();
+    const float inv = __fdiv_rn(1.0f, sqrtf(__fadd_rn(__fdiv_rn(s_tot, (float)d), rms_eps)));
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+        const int i = 4 * (tid + 256 * u);
+        if (i >= d) continue;
+        const float4 w = __ldg(reinterpret_cast<const float4 *>(norm_w + i));
+        float4 o;
+        o.x = bf16_round(__fmul_rn(w.x, __fmul_rn(acc[u].x, inv))); o.y = bf16_round(__fmul_rn(w.y, __fmul_rn(acc[u].y, inv)));
+        o.z = bf16_round(__fmul_rn(w.z, __fmul_rn(acc[u].z, inv))); o.w = bf16_round(__fmul_rn(w.w, __fmul_rn(acc[u].w, inv)));
+        *reinterpret_cast<float4 *>(y_normed + (size_t)row * d + i) = o;
+    }
+}
+
 // Y[j,i] = bf16(post[j]*f[i] + sum_k comb[k,j]*R[k,i]) (reference c/mhc.h:259-270,
 // c/layer.h:445-456).
+// Four adjacent channels per thread (16-byte loads and stores; all n + 1 loads of a thread are in flight together):
+// bound by HBM at many rows, (2 n + 1) * d * 4 bytes per row.  B200, 2,048 rows of
+// 4 x 4096: 136 -> 40 us, 7.5 TB/s out of L2 and HBM.  The scalar form takes the other shapes.
+template <int N>
+__global__ void __launch_bounds__(128)
+mhc_post4_kernel(const float *__restrict__ f, const float *__restrict__ res, const float *__restrict__ post,
+                 const float *__restrict__ comb, float *__restrict__ y4, int d) {
+    APUS_PDL_WAIT();
+    APUS_PDL_GO();
+    const int row = blockIdx.y, i = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= d) return;
+    const float *R = res + (size_t)row * N * d;
+    const float4 fv = *reinterpret_cast<const float4 *>(f + (size_t)row * d + i);
+    float4 rv[N];
+#pragma unroll
+    for (int k = 0; k < N; k++) rv[k] = *reinterpret_cast<const float4 *>(R + (size_t)k * d + i);
+    float po[N], cb[N * N];
+#pragma unroll
+    for (int k = 0; k < N; k++) po[k] = post[(size_t)row * N + k];
+#pragma unroll
+    for (int k = 0; k < N * N; k++) cb[k] = comb[(size_t)row * N * N + k];
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        float4 a = make_float4(__fmul_rn(po[j], fv.x), __fmul_rn(po[j], fv.y), __fmul_rn(po[j], fv.z), __fmul_rn(po[j], fv.w));
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            const float c = cb[k * N + j];
+            a.x = __fadd_rn(a.x, __fmul_rn(c, rv[k].x)); a.y = __fadd_rn(a.y, __fmul_rn(c, rv[k].y));
+            a.z = __fadd_rn(a.z, __fmul_rn(c, rv[k].z)); a.w = __fadd_rn(a.w, __fmul_rn(c, rv[k].w));
+        }
+        *reinterpret_cast<float4 *>(y4 + ((size_t)row * N + j) * d + i) =
+            make_float4(bf16_round(a.x), bf16_round(a.y), bf16_round(a.z), bf16_round(a.w));
+    }
+}
+
 __global__ void mhc_post_kernel(const float *__restrict__ f, const float *__restrict__ res,
                                 const float *__restrict__ post, const float *__restrict__ comb,
                                 float *__restrict__ y4, int d, int n) {
@@ -515,6 +670,12 @@ static float *ensure_raw(size_t floats, float *callers) {
 // raw[row, 0..nmix] for `rows` tokens in the sum order now in force.
 static int launch_mix(const float *x4, const float *fn, int nx, int nmix, float *raw, int rows,
                       cudaStream_t st) {
+    if (sum_tree(APUS_CUDA_TREE_MHC_MAPS) && rows >= 256) {      // a CTA per 8 rows still fills the SMs
+        launch_k(mhc_mix_rows_kernel<8, 5>, dim3((unsigned)ceil_div(nmix + 1, 5), (unsigned)ceil_div(rows, 8)), 256, 0, st, x4, fn, nx,
+                 nmix, rows, raw);
+        APUS_LAUNCHED();
+        return 0;
+    }
     if (sum_tree(APUS_CUDA_TREE_MHC_MAPS)) {
         launch_k(mhc_mix_kernel, dim3(nmix + 1, rows), 256, 0, st, x4, fn, nx, nmix, raw);
         APUS_LAUNCHED();
@@ -554,6 +715,13 @@ static int launch_finish(const float *x4, const float *raw, int d, int n, int nm
                          int *codes_written = nullptr) {
     if (codes_written) *codes_written = 0;
     if (d % 4 == 0 && n * n <= 32 && y && (size_t)d * sizeof(float) <= 48 * 1024) {
+        const bool aligned = (((uintptr_t)x4 | (uintptr_t)y | (uintptr_t)y_normed | (uintptr_t)norm_w) & 15) == 0;
+        if (finish_seq() && !xq && rows >= 512 && d <= 4096 && aligned) {     // a wave of CTAs and more, four words per thread
+            launch_k(mhc_pre_finish_rows_kernel<4>, rows, 256, (size_t)d * sizeof(float), st, x4, raw, d, n, nmix, scale, head_scale,
+                     base, norm_eps, hc_eps, iters, head_mode, norm_w, rms_eps, pre, post, comb, y, y_normed);
+            APUS_LAUNCHED();
+            return 0;
+        }
         // codes beside the normalised row when a CTA's slice (d / MHC_CL) is a whole number of 128-groups
         const bool codes = xq && xs && y_normed && d % (MHC_CL * 128) == 0;
         launch_k(mhc_pre_finish_cl_kernel, rows * MHC_CL, 128, finish_smem(d), st, x4, raw, d, n, nmix, scale, head_scale, base,
@@ -602,7 +770,10 @@ int mhc_post(const float *f, const float *res4, const float *post,
              cudaStream_t st) {
     APUS_REQUIRE(n >= 1 && n <= MHC_MAX_N, "mhc: n=%d unsupported", n);
     if (rows <= 0) return 0;
-    launch_k(mhc_post_kernel, dim3(ceil_div(d, 256), rows), 256, 0, st, f, res4, post, comb, y4, d, n);
+    if (n == 4 && d % 4 == 0 && (((uintptr_t)f | (uintptr_t)res4 | (uintptr_t)y4) & 15) == 0)
+        launch_k(mhc_post4_kernel<4>, dim3(ceil_div(d, 512), rows), 128, 0, st, f, res4, post, comb, y4, d);
+    else
+        launch_k(mhc_post_kernel, dim3(ceil_div(d, 256), rows), 256, 0, st, f, res4, post, comb, y4, d, n);
     APUS_LAUNCHED();
     return 0;
 }

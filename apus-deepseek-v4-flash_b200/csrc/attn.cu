@@ -486,12 +486,6 @@ sparse_pv_kernel(const float *__restrict__ sc, const float *__restrict__ sink, i
 #define SS_ROWB 128                       // bytes of a KV row staged per chunk: 64 BF16 or 32 f32 values of k
 #define SS_PITCHW 36                      // row pitch of the staged tile in 32-bit words (128 B + 16 B pad)
 
-__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool valid) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    const int sz = valid ? 16 : 0;        // 0: the 16 bytes are zero-filled
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(sz) : "memory");
-}
-
 // Scores.  A warp owns 16 heads x 8 NB candidates; lane = (hg, jg) owns heads 4hg..4hg+3 and candidates
 // jg, jg+8, ... (NB of them: 4 where the launch fills the GPU anyway; 1 for the few rows of a small step,
 // whose duration is one warp's instruction stream -- a quarter of it per warp and four times the warps).  The warp's 32 gathered rows are staged 128 bytes of k at a time in their

@@ -212,6 +212,61 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
+// ---- two f32 values per instruction ------------------------------------------------------------
+// A pair of f32 in one 64-bit register; each half is multiplied, added or fused exactly as the scalar
+// instruction would, so a kernel that walks two independent sums side by side keeps every bit while it
+// issues half the instructions.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+// acc + x * y per half: one rounding (FUSED; only where the product is exact, see below), or two
+template <bool FUSED>
+__device__ __forceinline__ f32x2 mac2(f32x2 acc, f32x2 x, f32x2 y) {
+    if (FUSED) {
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(y));
+    } else {
+        // scalar on purpose: a packed multiply followed by a packed add comes out of the compiler as one
+        // fused instruction, whatever the rounding modifiers say
+        const float2 a = unpack2(acc), u = unpack2(x), v = unpack2(y);
+        acc = pack2(__fadd_rn(a.x, __fmul_rn(u.x, v.x)), __fadd_rn(a.y, __fmul_rn(u.y, v.y)));
+    }
+    return acc;
+}
+
+// A product of two BF16 values (8 significant bits each) is exact in f32 as long as it neither overflows nor
+// leaves the normal range, and then fma(x, y, acc) is what the separate multiply and add return.  Both
+// operands +-0 or a BF16 value with 2^-60 <= |v| < 2^60 (biased exponent in [67, 187)) is enough.
+__device__ __forceinline__ bool fma_ok_f32(float v) {
+    const uint32_t u = __float_as_uint(v), a = u & 0x7fffffffu;
+    return a == 0u || ((u & 0xffffu) == 0u && a - (67u << 23) < (120u << 23));
+}
+// The same test on two BF16 values at once, per 16-bit half h = |value| bits: with
+// bit 15 set first no subtraction borrows across the halves, and bit 15 of
+// (h | 0x8000) - c then says h >= c.  Returns bit 15 / 31 set for a half that is
+// neither zero nor inside the window.
+__device__ __forceinline__ uint32_t fma_bad_bf16x2(uint32_t p) {
+    const uint32_t a = (p & 0x7fff7fffu) | 0x80008000u;
+    const uint32_t ge_lo = a - 0x21802180u;              // 67 << 7
+    const uint32_t ge_hi = a - 0x5d805d80u;              // 187 << 7
+    const uint32_t nz = a - 0x00010001u;
+    return nz & ~(ge_lo & ~ge_hi);
+}
+
+// 16-byte asynchronous copy into shared memory; an invalid one zero-fills (src must still be a mapped address)
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool valid) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    const int bytes = valid ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+
 static inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace apus

@@ -269,135 +269,169 @@ gemm_tc8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                      : "memory");
 }
 
-// ---- many activation rows (prefill / large batches): 128 rows per CTA -----------------------
-// Same structure with MMA N = 128: one weight tile is read once per 128
-// activation rows instead of once per 32, two accumulators of 128 TMEM columns,
-// and every fold thread keeps 128 running sums (its output row against the
-// CTA's 128 activation rows).  The fold (3 CUDA-core operations per element per
-// block: scale product, multiply, add -- the reference's order) costs more issue
-// slots than the block's MMAs, so this kernel is bound by the FP32 pipe at about
-// two thirds of the tensor peak; the per-block promotion is what keeps the
-// result equal to the reference's block-ordered f32 fold.
-constexpr int T8W_N = 128, T8W_NS = 5, T8W_NACC = 2;
+// ---- many activation rows (prefill / large batches): 128 rows per tile ----------------------
+// Same fold with MMA N = 128: one weight tile is read once per 128 activation rows.  A persistent CTA per SM
+// walks the 128 x 128 output tiles (output rows fastest, so that the CTAs of a moment share the activation
+// rows); the rings of stages and accumulators run on from tile to tile, so a tile's fill and its stores hide
+// behind its neighbour's MMAs:
+//   warps 0-7   fold: warp w owns output rows 32 (w % 4) .. and activation rows 64 (w / 4) .. of the tile, a
+//               thread one output row x 64 activation rows (32 pairs of running sums)
+//   warp 8      TMA producer (weight tile + activation tile per 128-wide block of K)
+//   warp 9      MMA issuer, four accumulators of 128 TMEM columns; owns the allocation
+//   warp 10     scales: per block the 128 products as[m, kb] * 2^(ws[kb] - 127), once for the whole tile
+// The fold of a block is dot * s added to the running sum, s the scale product.  s is a power of two, so with
+// 2^-100 <= s <= 2^90 (or s = 0, a row past the end) the multiplication is exact: dots are multiples of 2^-18
+// below 2^25.  One fused multiply-add then gives the sum the separate multiply and add give, and two of them go
+// into one instruction (f32x2): 32 instructions per thread and block where there were 384.  The scale warp
+// looks at every product; a block with one outside the window takes the two-instruction fold.
+// Bound by the tiles' way from L2: 32 KB per block, 128 flop per byte.  B200, 4096^3: 219 -> 151 us, 910 TFLOP/s.
+constexpr int T8W_N = 128, T8W_NS = 6, T8W_NACC = 4, T8W_THREADS = 352;
+constexpr int T8W_STAGE = T8_A_BYTES + T8W_N * 128;
 
 __device__ __forceinline__ uint32_t idesc_f8_wide() {
     return (1u << 4) | ((uint32_t)(T8W_N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
-__global__ void __launch_bounds__(T8_THREADS, 1)
+template <bool FUSED>
+__device__ __forceinline__ void fold_wide(f32x2 (&acc)[32], const uint32_t (&d0)[32], const uint32_t (&d1)[32], const float *sw) {
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        const ulonglong2 s = *reinterpret_cast<const ulonglong2 *>(sw + 4 * i);
+        const uint32_t *d = i < 8 ? d0 + 4 * i : d1 + 4 * (i - 8);
+        acc[2 * i] = mac2<FUSED>(acc[2 * i], pack2(__uint_as_float(d[0]), __uint_as_float(d[1])), s.x);
+        acc[2 * i + 1] = mac2<FUSED>(acc[2 * i + 1], pack2(__uint_as_float(d[2]), __uint_as_float(d[3])), s.y);
+    }
+}
+
+__global__ void __launch_bounds__(T8W_THREADS, 1)
 gemm_tc8_wide_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_x,
                      const Tc8Args a) {
     APUS_PDL_WAIT();
     APUS_PDL_GO();
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    constexpr int B_BYTES = T8W_N * 128, STAGE = T8_A_BYTES + B_BYTES, NS = T8W_NS, NACC = T8W_NACC;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + (size_t)NS * STAGE);
-    uint64_t *full = bars, *empty = bars + NS, *acc_full = bars + 2 * NS, *acc_empty = bars + 2 * NS + NACC;
-    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(bars + 2 * NS + 2 * NACC);
+    constexpr int STAGE = T8W_STAGE, NS = T8W_NS, NACC = T8W_NACC;
+    float *s_sw = reinterpret_cast<float *>(smem + (size_t)NS * STAGE);          // [NACC][128] scale products
+    uint64_t *bars = reinterpret_cast<uint64_t *>(s_sw + NACC * T8W_N);
+    uint64_t *full = bars, *empty = bars + NS, *acc_full = bars + 2 * NS, *acc_empty = acc_full + NACC, *sw_full = acc_empty + NACC;
+    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(sw_full + NACC);
     volatile int *s_abort = reinterpret_cast<volatile int *>(s_tmem + 1);
-    float *s_as = reinterpret_cast<float *>(s_tmem + 4);          // [NC][128] activation scales
+    volatile int *s_ok = reinterpret_cast<volatile int *>(s_tmem + 2);           // [NACC] the block's scales are in the window
     const int K = a.K, O = a.O, NC = K >> 7, M = a.M;
-    float *s_ws = s_as + (size_t)NC * T8W_N;                       // [NC] weight tile scales
-    const int row0 = (int)blockIdx.y * T8W_N;
-    const int nrows = min(T8W_N, M - row0);
-    if (nrows <= 0) return;
+    const int n_o = O >> 7, tiles = n_o * ((M + T8W_N - 1) / T8W_N);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int tile_row = (int)blockIdx.x * 128;
 
     if (tid == 0) {
         for (int s = 0; s < NS; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < NACC; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 128); }
+        for (int b = 0; b < NACC; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); mbar_init(&sw_full[b], 1); }
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 5) {
+    if (warp == 9) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(s_tmem)), "r"(NACC * T8W_N) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    if (tid < 128) {
-        for (int i = tid; i < NC * T8W_N; i += 128) {
-            const int kb = i / T8W_N, n = i - kb * T8W_N;
-            s_as[i] = n < nrows ? a.ascales[(size_t)(row0 + n) * NC + kb] : 0.f;
-        }
-        const uint8_t *wsa = a.scales_a + (size_t)blockIdx.x * NC;
-        for (int i = tid; i < NC; i += 128) s_ws[i] = ue8m0_f32(wsa[i]);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *s_tmem;
     int fail = 0;
+    uint32_t it = 0;                                   // blocks of this CTA so far: ring positions and phases
 
-    if (warp == 4) {
+    if (warp == 8) {
         if (lane == 0) {
-            for (int i = 0; i < NC && !fail; i++) {
-                const int s = i % NS;
-                const uint32_t ph = (uint32_t)(i / NS) & 1u;
-                if (!mbar_wait(&empty[s], ph ^ 1u, s_abort)) { fail = 11; break; }
-                uint8_t *st = smem + (size_t)s * STAGE;
-                mbar_expect_tx(&full[s], STAGE);
-                tma_load_2d(st, &tm_a, i * 128, tile_row, &full[s]);
-                tma_load_2d(st + T8_A_BYTES, &tm_x, i * 128, row0, &full[s]);
+            for (int tile = blockIdx.x; tile < tiles && !fail; tile += gridDim.x) {
+                const int o0 = (tile % n_o) * 128, row0 = (tile / n_o) * T8W_N;
+                for (int i = 0; i < NC; i++, it++) {
+                    const uint32_t s = it % NS, ph = (it / NS) & 1u;
+                    if (!mbar_wait(&empty[s], ph ^ 1u, s_abort)) { fail = 11; break; }
+                    uint8_t *st = smem + (size_t)s * STAGE;
+                    mbar_expect_tx(&full[s], STAGE);
+                    tma_load_2d(st, &tm_a, i * 128, o0, &full[s]);
+                    tma_load_2d(st + T8_A_BYTES, &tm_x, i * 128, row0, &full[s]);
+                }
             }
         }
-    } else if (warp == 5) {
+    } else if (warp == 9) {
         if (lane == 0) {
             const uint32_t idesc = idesc_f8_wide();
-            for (int i = 0; i < NC && !fail; i++) {
-                const int s = i % NS, b = i % NACC;
-                const uint32_t ph = (uint32_t)(i / NS) & 1u, pb = (uint32_t)(i / NACC) & 1u;
-                if (!mbar_wait(&acc_empty[b], pb ^ 1u, s_abort)) { fail = 12; break; }
-                if (!mbar_wait(&full[s], ph, s_abort)) { fail = 13; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t sa = smem_u32(smem + (size_t)s * STAGE);
-                const uint64_t da = umma_desc_sw128(sa), dx = umma_desc_sw128(sa + T8_A_BYTES);
+            for (int tile = blockIdx.x; tile < tiles && !fail; tile += gridDim.x) {
+                for (int i = 0; i < NC; i++, it++) {
+                    const uint32_t s = it % NS, ph = (it / NS) & 1u, b = it % NACC, pb = (it / NACC) & 1u;
+                    if (!mbar_wait(&acc_empty[b], pb ^ 1u, s_abort)) { fail = 12; break; }
+                    if (!mbar_wait(&full[s], ph, s_abort)) { fail = 13; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t sa = smem_u32(smem + (size_t)s * STAGE);
+                    const uint64_t da = umma_desc_sw128(sa), dx = umma_desc_sw128(sa + T8_A_BYTES);
 #pragma unroll
-                for (int j = 0; j < 4; j++) umma_f8(tmem + b * T8W_N, da + 2 * j, dx + 2 * j, idesc, j ? 1u : 0u);
-                umma_commit(&empty[s]);
-                umma_commit(&acc_full[b]);
+                    for (int j = 0; j < 4; j++) umma_f8(tmem + b * T8W_N, da + 2 * j, dx + 2 * j, idesc, j ? 1u : 0u);
+                    umma_commit(&empty[s]);
+                    umma_commit(&acc_full[b]);
+                }
+            }
+        }
+    } else if (warp == 10) {
+        // lane l: activation rows 4 l .. 4 l + 3 of the tile; the next block's scales are read while this one's wait
+        float as[4], nx[4];
+        for (int tile = blockIdx.x; tile < tiles && !fail; tile += gridDim.x) {
+            const int row0 = (tile / n_o) * T8W_N, nrows = min(T8W_N, M - row0);
+            const uint8_t *wsa = a.scales_a + (size_t)(tile % n_o) * NC;
+            const float *src = a.ascales + (size_t)(row0 + 4 * lane) * NC;
+            auto load = [&](int i, float (&v)[4]) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) v[j] = 4 * lane + j < nrows ? __ldg(src + (size_t)j * NC + i) : 0.f;
+            };
+            load(0, as);
+            for (int i = 0; i < NC; i++, it++) {
+                const uint32_t b = it % NACC, pb = (it / NACC) & 1u;
+                if (i + 1 < NC) load(i + 1, nx);
+                const float ws = ue8m0_f32(__ldg(wsa + i));
+                // the lanes leave together: the votes here and the tensor-memory loads below are for whole warps
+                if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[b], pb ^ 1u, s_abort))) { fail = 15; break; }
+                bool ok = true;
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    as[j] = __fmul_rn(as[j], ws);
+                    ok = ok && (as[j] == 0.f || (as[j] >= 7.88860905e-31f && as[j] <= 1.23794004e27f));     // 2^-100, 2^90
+                }
+                *reinterpret_cast<float4 *>(s_sw + b * T8W_N + 4 * lane) = make_float4(as[0], as[1], as[2], as[3]);
+                const int all = __all_sync(0xffffffffu, ok);
+                if (lane == 0) s_ok[b] = all;
+                mbar_arrive_warp(&sw_full[b], lane);
+#pragma unroll
+                for (int j = 0; j < 4; j++) as[j] = nx[j];
             }
         }
     } else {
-        const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
-        float acc[T8W_N];
+        const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16, col0 = (uint32_t)(warp >> 2) * 64;
+        for (int tile = blockIdx.x; tile < tiles && !fail; tile += gridDim.x) {
+            f32x2 acc[32];
 #pragma unroll
-        for (int n = 0; n < T8W_N; n++) acc[n] = 0.f;
-        for (int i = 0; i < NC && !fail; i++) {
-            const int b = i % NACC;
-            const uint32_t pb = (uint32_t)(i / NACC) & 1u;
-            if (!mbar_wait(&acc_full[b], pb, s_abort)) { fail = 14; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const float ws = s_ws[i];
-            const float4 *as4 = reinterpret_cast<const float4 *>(s_as + (size_t)i * T8W_N);
-#pragma unroll
-            for (int qd = 0; qd < T8W_N / 32; qd++) {
-                uint32_t d[32];
-                tmem_ld32(tmem + lane_base + b * T8W_N + qd * 32, d);
+            for (int n = 0; n < 32; n++) acc[n] = 0ull;
+            for (int i = 0; i < NC; i++, it++) {
+                const uint32_t b = it % NACC, pb = (it / NACC) & 1u;
+                const bool there = mbar_wait(&sw_full[b], pb, s_abort) && mbar_wait(&acc_full[b], pb, s_abort);
+                if (!__all_sync(0xffffffffu, there)) { fail = 14; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                uint32_t d0[32], d1[32];
+                tmem_ld32(tmem + lane_base + b * T8W_N + col0, d0);
+                tmem_ld32(tmem + lane_base + b * T8W_N + col0 + 32, d1);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (qd == T8W_N / 32 - 1) {              // the accumulator has been read completely
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    mbar_arrive(&acc_empty[b]);
-                }
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    const float4 s4 = as4[qd * 8 + q];
-                    const float sv[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-                    for (int r = 0; r < 4; r++) {
-                        const int n = qd * 32 + 4 * q + r;
-                        acc[n] = __fadd_rn(acc[n], __fmul_rn(__uint_as_float(d[4 * q + r]), __fmul_rn(sv[r], ws)));
-                    }
-                }
+                const float *sw = s_sw + b * T8W_N + col0;
+                if (s_ok[b]) fold_wide<true>(acc, d0, d1, sw);
+                else fold_wide<false>(acc, d0, d1, sw);
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                mbar_arrive_warp(&acc_empty[b], lane); // the accumulator and its scales have been read
             }
-        }
-        if (!fail) {
-            const int o = tile_row + tid;
-            if (o < O) {
+            if (fail) break;
+            const int row0 = (tile / n_o) * T8W_N + (int)col0, nrows = min(64, M - row0);
+            float *out = a.out + (size_t)row0 * O + (size_t)(tile % n_o) * 128 + (warp & 3) * 32 + lane;
 #pragma unroll
-                for (int n = 0; n < T8W_N; n++)
-                    if (n < nrows) a.out[(size_t)(row0 + n) * O + o] = a.round_out ? bf16_round(acc[n]) : acc[n];
+            for (int n = 0; n < 64; n++) {
+                const float2 v2 = unpack2(acc[n >> 1]);
+                const float v = n & 1 ? v2.y : v2.x;
+                if (n < nrows) out[(size_t)n * O] = a.round_out ? bf16_round(v) : v;
             }
         }
     }
@@ -408,7 +442,7 @@ gemm_tc8_wide_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 5)
+    if (warp == 9)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NACC * T8W_N)
                      : "memory");
 }
@@ -451,12 +485,14 @@ int gemm_tc8_wide(const Tc8Args &a, cudaStream_t st) {
     APUS_REQUIRE(a.K % 128 == 0 && a.K <= 128 * 64 && a.O % 128 == 0 && !a.pair,
                  "gemm_tc8_wide: unsupported shape O=%d K=%d", a.O, a.K);
     if (a.M <= 0) return 0;
-    const int NC = a.K >> 7;
-    const size_t smem = (size_t)T8W_NS * (T8_A_BYTES + T8W_N * 128) + 1024 + 256 + (size_t)NC * T8W_N * 4 + (size_t)NC * 4;
-    if (ensure_dyn_smem((const void *)gemm_tc8_wide_kernel, 224 * 1024)) return 1;
-    dim3 grid((unsigned)(a.O / 128), (unsigned)((a.M + T8W_N - 1) / T8W_N));
-    launch_k(gemm_tc8_wide_kernel, grid, T8_THREADS, smem, st, *reinterpret_cast<const CUtensorMap *>(a.map_a),
-                                                         *reinterpret_cast<const CUtensorMap *>(a.map_x), a);
+    const size_t smem = (size_t)T8W_NS * T8W_STAGE + T8W_NACC * T8W_N * 4 + 1024 + 256;
+    if (ensure_dyn_smem((const void *)gemm_tc8_wide_kernel, smem)) return 1;
+    int dev = 0, sms = 0;
+    APUS_CUDA_OK(cudaGetDevice(&dev));
+    APUS_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const long long tiles = (long long)(a.O / 128) * ((a.M + T8W_N - 1) / T8W_N);
+    launch_k(gemm_tc8_wide_kernel, (unsigned)(tiles < sms ? tiles : sms), T8W_THREADS, smem, st,
+             *reinterpret_cast<const CUtensorMap *>(a.map_a), *reinterpret_cast<const CUtensorMap *>(a.map_x), a);
     APUS_LAUNCHED();
     return 0;
 }

@@ -143,29 +143,6 @@ struct SeqCfg {
     static constexpr int SMEM = NST * STAGE + 2 * WIDE + 16;   // ring, two widened halves, the tiles' exactness flags
 };
 
-__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool valid) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    const int bytes = valid ? 16 : 0;                    // 0 source bytes = zero fill
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
-}
-
-// +-0, or a BF16 value with 67 <= biased exponent < 187
-__device__ __forceinline__ bool fma_ok_f32(float v) {
-    const uint32_t u = __float_as_uint(v), a = u & 0x7fffffffu;
-    return a == 0u || ((u & 0xffffu) == 0u && a - (67u << 23) < (120u << 23));
-}
-// The same test on two BF16 values at once, per 16-bit half h = |value| bits: with
-// bit 15 set first no subtraction borrows across the halves, and bit 15 of
-// (h | 0x8000) - c then says h >= c.  Returns bit 15 / 31 set for a half that is
-// neither zero nor inside the window.
-__device__ __forceinline__ uint32_t fma_bad_bf16x2(uint32_t p) {
-    const uint32_t a = (p & 0x7fff7fffu) | 0x80008000u;
-    const uint32_t ge_lo = a - 0x21802180u;              // 67 << 7
-    const uint32_t ge_hi = a - 0x5d805d80u;              // 187 << 7
-    const uint32_t nz = a - 0x00010001u;
-    return nz & ~(ge_lo & ~ge_hi);
-}
-
 // Eight consecutive k of one output row against one token: acc = acc + x*w, k ascending.
 template <bool FUSED>
 __device__ __forceinline__ float seq_walk8(float a, const float4 &wa, const float4 &wb, const float4 &xa,

@@ -32,6 +32,12 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// One arrival for a whole warp (converged): arrivals at one barrier are served one after another, so a barrier
+// that every thread of a CTA arrives at costs the hand-over some four cycles per thread.
+__device__ __forceinline__ void mbar_arrive_warp(uint64_t *bar, int lane) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+}
 // Bounded wait for the phase with the given parity; false on expiry or abort.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
     unsigned long long t0 = 0;

@@ -3,10 +3,28 @@ kernel of this library that knows no tiles."""
 import numpy as np
 import pytest
 
-from _gpu import bits, cuda_moe
+from _gpu import bits, cuda_moe, cuda_qgemm
 from apus_b200 import synth
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,O,K", [(64, 128, 128), (65, 256, 384), (127, 128, 1024), (129, 384, 256), (260, 4096, 640),
+                                   (1200, 2048, 512)])
+@pytest.mark.parametrize("scales", ["usual", "extreme"])
+def test_fp8_wide_rows_equal_narrow_rows(M, O, K, scales):
+    rng = np.random.default_rng(M + K)
+    code = lambda *s: rng.integers(0, 127, s).astype(np.uint8) | (rng.integers(0, 2, s).astype(np.uint8) << 7)   # noqa: E731
+    codes, acodes = code(O, K), code(M, K)
+    ws = rng.integers(119, 122, (O // 128, K // 128)).astype(np.uint8)
+    asc = np.exp2(rng.integers(-12, 3, (M, K // 128))).astype(np.float32)
+    if scales == "extreme":                      # scale products outside the window of the one-rounding fold
+        ws.flat[:: 2] = 0
+        ws.flat[1:: 5] = 20
+        asc[:: 3] = np.float32(2.0 ** -22)
+    got = cuda_qgemm(8, codes, ws, acodes, asc, O)
+    want = np.concatenate([cuda_qgemm(8, codes, ws, acodes[i:i + 32], asc[i:i + 32], O) for i in range(0, M, 32)])
+    assert np.array_equal(bits(got), bits(want))
 
 
 @pytest.mark.parametrize("T", [33, 513, 2100])

@@ -115,6 +115,7 @@ struct TcbfArgs {
     int out_ld, round_out;
     float *out;                          // [M, out_ld]
     int ksplit;                          // K chunks (tcbf_ksplit); > 1 needs part + counters
+    int wide;                            // map_x has 128-row boxes: the 128-row kernel (tcbf_wide)
     float *part;                         // [ksplit, M, batch*O] scratch
     int *counters;                       // zeroed, one per (output tile, row group); left zeroed
     uint8_t *q_out;                      // ksplit > 1, out_ld % 128 == 0: also the E4M3 activation codes [M, out_ld] ...
@@ -124,7 +125,8 @@ int gemm_tcbf(const TcbfArgs &a, cudaStream_t st);
 int gemm_tcbf_status(int reset);
 int tcbf_ksplit(int O, int K, int batch, int M);
 int tcbf_make_weight_map(void *out_map, const void *w_bf16, long long rows, int K);
-int tcbf_make_act_map(void *out_map, const void *x_bf16, long long rows, long long cols);
+bool tcbf_wide(int M, int S);             // M rows with S K chunks go to the 128-row tiles (no scratch, no codes)
+int tcbf_make_act_map(void *out_map, const void *x_bf16, long long rows, long long cols, bool wide);
 int f32_to_bf16(const float *x, uint16_t *y, long long n, cudaStream_t st);
 // Scratch memory that belongs to a stream (launches on one stream run one after another, so
 // they may share it): `bytes` of workspace and, separately, `n_counters` ints that are zero

@@ -433,7 +433,8 @@ static int linear_tcbf(const void *w, const float *x, int x_koff, int x_ld, floa
                        int K, int O, int flags, cudaStream_t st, LinCodes *codes) {
     const int S = tcbf_ksplit(O, K, batch, M);
     const size_t xb = (((size_t)M * x_ld * 2) + 255) & ~(size_t)255;
-    const size_t pb = S > 1 ? (size_t)S * M * batch * O * 4 : 0;
+    const bool wide = !codes && tcbf_wide(M, S);
+    const size_t pb = S > 1 && !wide ? (size_t)S * M * batch * O * 4 : 0;
     const size_t n_cnt = (size_t)(O / 128) * batch * ((M + 31) / 32);
     void *ws = nullptr;
     int *cnt = nullptr;
@@ -441,9 +442,9 @@ static int linear_tcbf(const void *w, const float *x, int x_koff, int x_ld, floa
     uint16_t *xh = (uint16_t *)ws;
     if (f32_to_bf16(x, xh, (long long)M * x_ld, st)) return 1;
     alignas(64) unsigned char map_w[128], map_x[128];
-    if (tcbf_make_weight_map(map_w, w, (long long)batch * O, K) || tcbf_make_act_map(map_x, xh, M, x_ld)) return 1;
+    if (tcbf_make_weight_map(map_w, w, (long long)batch * O, K) || tcbf_make_act_map(map_x, xh, M, x_ld, wide)) return 1;
     TcbfArgs a = {};
-    a.map_w = map_w; a.map_x = map_x;
+    a.map_w = map_w; a.map_x = map_x; a.wide = wide ? 1 : 0;
     a.M = M; a.O = O; a.K = K; a.batch = batch; a.x_koff = x_koff;
     a.out_ld = out_ld; a.round_out = (flags & APUS_CUDA_R_OUT) ? 1 : 0; a.out = out;
     a.ksplit = S; a.part = (float *)((char *)ws + xb); a.counters = cnt;

@@ -267,6 +267,17 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src, bool vali
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
 }
 
+// The experts' activation (reference c/moe.h:126-146): BF16-rounded gate and up, clamped, g * sigmoid(g) * u.
+__device__ __forceinline__ float swiglu(float gate, float up, float limit) {
+    float g = bf16_round(gate), u = bf16_round(up);
+    if (limit > 0.f) {
+        u = fminf(fmaxf(u, -limit), limit);
+        g = fminf(g, limit);
+    }
+    float sig = 1.0f / (1.0f + exp_rn(-g));
+    return bf16_round(__fmul_rn(__fmul_rn(g, sig), u));
+}
+
 static inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace apus

@@ -57,16 +57,6 @@ __device__ __forceinline__ void fp4_expand(uint32_t w, uint32_t &lo, uint32_t &h
     hi = __byte_perm(T0, T1, m >> 16) | ((w << 4) & 0x80808080u);
 }
 
-__device__ __forceinline__ float swiglu(float gate, float up, float limit) {
-    float g = bf16_round(gate), u = bf16_round(up);
-    if (limit > 0.f) {
-        u = fminf(fmaxf(u, -limit), limit);
-        g = fminf(g, limit);
-    }
-    float sig = 1.0f / (1.0f + exp_rn(-g));
-    return bf16_round(__fmul_rn(__fmul_rn(g, sig), u));
-}
-
 template <bool ZS>
 __device__ __forceinline__ float wscale(uint32_t word, int b) {
     uint32_t byte = (word >> (8 * b)) & 0xffu;

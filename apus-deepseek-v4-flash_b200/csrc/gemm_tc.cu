@@ -60,16 +60,6 @@ __device__ __forceinline__ void umma_mxf8f6f4(uint32_t d_tmem, uint64_t adesc, u
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
         : "memory");
 }
-__device__ __forceinline__ float swiglu_tc(float gate, float up, float limit) {
-    float g = bf16_round(gate), u = bf16_round(up);
-    if (limit > 0.f) {
-        u = fminf(fmaxf(u, -limit), limit);
-        g = fminf(g, limit);
-    }
-    float sig = 1.0f / (1.0f + exp_rn(-g));
-    return bf16_round(__fmul_rn(__fmul_rn(g, sig), u));
-}
-
 template <bool PAIR, int NS>
 __global__ void __launch_bounds__(TC_THREADS, 2)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
@@ -226,7 +216,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
 #pragma unroll
                 for (int n = 0; n < TC_N; n++) {
                     if (n >= nrows) break;                 // a work item at decode sizes holds one to three rows
-                    hv[n] = swiglu_tc(__uint_as_float(d0[n]), __uint_as_float(d1[n]), a.limit);
+                    hv[n] = swiglu(__uint_as_float(d0[n]), __uint_as_float(d1[n]), a.limit);
                     const float m = warp_max(fabsf(hv[n]));
                     if (lane == 0) s_amax[warp * TC_N + n] = m;
                 }
@@ -248,7 +238,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                     if (n >= nrows) break;
                     const int dst = a.orow ? a.orow[row0 + n] : row0 + n;
                     float v;
-                    if (PAIR) v = swiglu_tc(__uint_as_float(d0[n]), __uint_as_float(d1[n]), a.limit);
+                    if (PAIR) v = swiglu(__uint_as_float(d0[n]), __uint_as_float(d1[n]), a.limit);
                     else v = a.round_out ? bf16_round(__uint_as_float(d0[n])) : __uint_as_float(d0[n]);
                     a.out[(size_t)dst * O + o] = v;
                 }
@@ -291,7 +281,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                 }
                 const int dst = a.orow ? a.orow[row0 + n] : row0 + n;
                 float v;
-                if (PAIR) v = swiglu_tc(va, vb, a.limit);
+                if (PAIR) v = swiglu(va, vb, a.limit);
                 else v = a.round_out ? bf16_round(va) : va;
                 a.out[(size_t)dst * O + o] = v;
             }

@@ -52,16 +52,6 @@ __device__ __forceinline__ void umma_f8(uint32_t d_tmem, uint64_t adesc, uint64_
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
-__device__ __forceinline__ float swiglu8(float gate, float up, float limit) {
-    float g = bf16_round(gate), u = bf16_round(up);
-    if (limit > 0.f) {
-        u = fminf(fmaxf(u, -limit), limit);
-        g = fminf(g, limit);
-    }
-    float sig = 1.0f / (1.0f + exp_rn(-g));
-    return bf16_round(__fmul_rn(__fmul_rn(g, sig), u));
-}
-
 template <bool PAIR, int NS>
 __global__ void __launch_bounds__(T8_THREADS, 2)
 gemm_tc8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
@@ -221,7 +211,7 @@ gemm_tc8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                 for (int n = 0; n < T8_N; n++) {
                     if (n >= nrows) break;
                     float v;
-                    if (PAIR) v = swiglu8(accA[n], accB[n], a.limit);
+                    if (PAIR) v = swiglu(accA[n], accB[n], a.limit);
                     else v = a.round_out ? bf16_round(accA[n]) : accA[n];
                     a.out[(size_t)(row0 + n) * O + o] = v;
                 }
@@ -254,7 +244,7 @@ gemm_tc8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
                     if (PAIR) vb = __fadd_rn(vb, __ldcg(a.part + ((size_t)(NC + c) * M + row0 + n) * O + o));
                 }
                 float v;
-                if (PAIR) v = swiglu8(va, vb, a.limit);
+                if (PAIR) v = swiglu(va, vb, a.limit);
                 else v = a.round_out ? bf16_round(va) : va;
                 a.out[(size_t)(row0 + n) * O + o] = v;
             }

@@ -24,6 +24,8 @@ int repack_fp8(const uint8_t *codes, int O, int K, uint8_t *out_codes,
 // arow (nullable) gathers input rows: row m is read from x[arow[m]].
 int act_quant(const float *x, const int *arow, int M, int K, uint8_t *codes,
               float *scales, const int *m_dev, cudaStream_t st);
+// codes [M, K] and scales [M, K / 128] of swiglu(gate, up), both [M, K]
+int swiglu_quant(const float *gate, const float *up, float limit, int M, int K, uint8_t *codes, float *scales, cudaStream_t st);
 // RMSNorm rows (reference c/attn.h:371-378).
 int rms_norm(const float *x, const float *w, float eps, float *y, int64_t n,
              int64_t rows, cudaStream_t st);

@@ -68,6 +68,36 @@ int act_quant(const float *x, const int *arow, int M, int K, uint8_t *codes,
     return 0;
 }
 
+// codes and scales of swiglu(gate, up) for the down projection: one warp per (row, 128-group), as above
+__global__ void __launch_bounds__(256)
+swiglu_quant_kernel(const float *__restrict__ gate, const float *__restrict__ up, float limit, long long groups,
+                    uint8_t *__restrict__ codes, float *__restrict__ scales) {
+    APUS_PDL_WAIT();
+    APUS_PDL_GO();
+    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (w >= groups) return;
+    const float4 g = *reinterpret_cast<const float4 *>(gate + w * 128 + lane * 4);
+    const float4 u = *reinterpret_cast<const float4 *>(up + w * 128 + lane * 4);
+    const float4 v = make_float4(swiglu(g.x, u.x, limit), swiglu(g.y, u.y, limit), swiglu(g.z, u.z, limit), swiglu(g.w, u.w, limit));
+    float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+    amax = fmaxf(warp_max(amax), 1e-4f);
+    const float s = ceil_pow2(__fmul_rn(amax, 1.0f / 448.0f));
+    const float inv = __uint_as_float(0x7f000000u - __float_as_uint(s));
+    const uint32_t lo = e4m3x2_from_f32(v.x * inv, v.y * inv), hi = e4m3x2_from_f32(v.z * inv, v.w * inv);
+    *reinterpret_cast<uint32_t *>(codes + w * 128 + lane * 4) = lo | (hi << 16);
+    if (lane == 0) scales[w] = s;
+}
+
+int swiglu_quant(const float *gate, const float *up, float limit, int M, int K, uint8_t *codes, float *scales, cudaStream_t st) {
+    APUS_REQUIRE(K % 128 == 0, "swiglu_quant: K=%d must be a multiple of 128", K);
+    if (M <= 0) return 0;
+    const long long groups = (long long)M * (K / 128);
+    launch_k(swiglu_quant_kernel, (unsigned)ceil_div(groups, 8), 256, 0, st, gate, up, limit, groups, codes, scales);
+    APUS_LAUNCHED();
+    return 0;
+}
+
 // One CTA per row: y = bf16(w * (x * 1/sqrt(mean(x^2)+eps))) (reference
 // c/attn.h:371-378).  seq: the sum of squares walks the row in index order with
 // one accumulator and rounded squares, as the reference's loop does; otherwise

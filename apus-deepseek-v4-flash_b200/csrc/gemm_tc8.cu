@@ -85,7 +85,7 @@ gemm_tc8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
 
     if (tid == 0) {
         for (int s = 0; s < NS; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < NACC; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 128); }
+        for (int b = 0; b < NACC; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4); }
         *s_abort = 0;
         *s_last = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -163,14 +163,15 @@ gemm_tc8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         for (int i = c0; i < c1 && !fail; i++) {
             const int b = (i - c0) % NACC;
             const uint32_t pb = (uint32_t)((i - c0) / NACC) & 1u;
-            if (!mbar_wait(&acc_full[b], pb, s_abort)) { fail = 14; break; }
+            // the lanes leave together: the tensor-memory loads and the arrival are for whole warps
+            if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[b], pb, s_abort))) { fail = 14; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             uint32_t d0[32], d1[32];
             tmem_ld32(tmem + lane_base + b * 32, d0);
             if (PAIR) tmem_ld32(tmem + lane_base + NACC * 32 + b * 32, d1);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            mbar_arrive(&acc_empty[b]);                // the tensor core may overwrite this accumulator
+            mbar_arrive_warp(&acc_empty[b], lane);     // the tensor core may overwrite this accumulator
             const float wsa = s_ws[i], wsb = PAIR ? s_ws[NC + i] : 0.f;
             const float4 *as4 = reinterpret_cast<const float4 *>(s_as + (size_t)i * T8_N);
             if (S > 1) {

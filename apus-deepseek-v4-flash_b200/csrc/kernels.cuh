@@ -78,6 +78,7 @@ struct TcArgs {
     const int *orow;                     // nullable: output row of sorted position p
     float *out;
     int tx_bytes;                        // 0 = default transaction bytes per stage
+    int rows64;                          // work items hold up to 64 rows, map_x has 64-row boxes (else 32)
     uint8_t *q_out;                      // pair mode, optional: write the outputs quantised for the next GEMM
     float *qs_out;                       //   (E4M3 codes [rows, O] + scales [rows, O/128], sorted order) instead of `out`
     int total_rows;                      // activation rows over all work items (0: unknown, K is never split)
@@ -88,7 +89,7 @@ struct TcArgs {
 int gemm_tc(const TcArgs &a, cudaStream_t st);
 int gemm_tc_status(int reset);
 int tc_make_weight_map(void *out_map, const void *codes, long long rows, int K);
-int tc_make_act_map(void *out_map, const void *codes, long long rows, int K);
+int tc_make_act_map(void *out_map, const void *codes, long long rows, int K, int box_rows = 32);
 
 // ---- tcgen05 FP8 GEMM on the reference weight storage (gemm_tc8.cu) -----------------------
 struct Tc8Args {

@@ -11,12 +11,26 @@ namespace apus {
 // Reference c/attn.h:668-687: k passes of strict-greater argmax over unused
 // entries, i.e. the k largest scores, equal scores ordered by ascending index,
 // emitted in that order.  Restated as a selection on the composite key
-// (score, -index): an 8-bit radix select on the order-preserving integer image
-// of the score finds the k-th largest score value T and how many scores are
-// strictly greater; a second, index-ordered sweep takes every score > T and
-// the lowest-index scores == T until k are chosen; a bitonic sort of the k
-// (key, index) pairs gives the output order.  One CTA per row.
-// Bytes per row: 5 sweeps over n*4 (L2-resident for n <= a few million).
+// (score, -index): a radix select on the order-preserving integer image of the
+// score finds the k-th largest score value, every score above it and the
+// lowest-index scores equal to it are collected, and a bitonic sort of the k
+// (key, index) pairs gives the output order.
+//
+// One CTA per row, or a cluster of eight for long rows: there every CTA
+// histograms its slice, all of them add their histograms into rank 0's shared
+// memory and derive the same digit from the sum, so no result has to be sent
+// around; the chosen entries are stored into rank 0's shared memory, where rank 0
+// sorts and writes them out.  Nobody touches another CTA's shared memory before a
+// first cluster barrier (a CTA of the cluster may not have started yet), and
+// nobody leaves before the last reader is done.
+//
+// The row crosses L2 once: a thread keeps its KPT keys in registers for every
+// pass (KPT = 0: rows too long for that are read again by each pass).  Digits of
+// 11, 11 and 10 bits; as soon as the bin that holds the k-th score is taken whole
+// no further digit is needed, which ends most rows after the second, and only a
+// tie at the boundary takes the index-ordered sweep.  The sort exchanges through
+// shuffles below a stride of 32.  Bound by the latency of these short phases.
+// B200: 262,144 scores, k = 512 83.6 -> 26.6 us; 32 rows of 2,048 14.7 -> 9.1 us.
 __device__ __forceinline__ uint32_t order_key(float f) {
     uint32_t u = __float_as_uint(f);
     if ((u << 1) == 0) u = 0;                 // -0.0 and +0.0 compare equal
@@ -26,270 +40,180 @@ __device__ __forceinline__ uint32_t order_key(float f) {
 #define TOPK_THREADS 1024
 #define TOPK_MAX_K 2048
 
-__global__ void __launch_bounds__(TOPK_THREADS)
+#define TOPK_CL 8
+#define TOPK_BINS 2048
+template <int CL, int KPT>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(TOPK_THREADS)
 topk_stable_kernel(const float *__restrict__ scores, int n, int k, int32_t *__restrict__ idx_out,
                    const long long *__restrict__ dyn_pos, int ratio, long long chunk_pos0, int rows_per_pos) {
     APUS_PDL_WAIT();
     APUS_PDL_GO();
-    __shared__ unsigned hist[256];
-    __shared__ unsigned s_prefix, s_need, s_greater, s_taken, s_base;
-    __shared__ unsigned long long sel[TOPK_MAX_K];
-    const float *row = scores + (size_t)blockIdx.x * n;     // n, k as given are the row strides
-    int32_t *out = idx_out + (size_t)blockIdx.x * k;
-    if (dyn_pos || rows_per_pos > 0) {                      // live sizes from the position (of the row, in a chunk)
-        const long long nbs = ((dyn_pos ? *dyn_pos : chunk_pos0 + blockIdx.x / rows_per_pos) + 1) / ratio;
-        n = (int)(nbs < n ? nbs : n);
-        k = k < n ? k : n;
-        if (k <= 0) return;
-    }
-    const int tid = threadIdx.x;
-
-    const int lane = tid & 31, warp = tid >> 5;
-    if (k >= n) {
-        // every score is selected (a row shorter than k: the first 4 k positions of a sequence): only the order is left
-        for (int i = tid; i < n; i += TOPK_THREADS)
-            sel[i] = ((unsigned long long)order_key(row[i]) << 32) | (0xffffffffu - (unsigned)i);
-        k = n;
-        __syncthreads();
-    } else {
-    // radix select: after the loop `prefix` is the key of the k-th largest score
-    if (tid == 0) { s_prefix = 0; s_need = (unsigned)k; s_greater = 0; }
-    for (int pass = 0; pass < 4; pass++) {
-        const int shift = 24 - 8 * pass;
-        for (int i = tid; i < 256; i += TOPK_THREADS) hist[i] = 0;
-        __syncthreads();
-        const unsigned prefix = s_prefix;
-        const unsigned himask = pass ? (0xffffffffu << (shift + 8)) : 0u;
-        for (int i = tid; i < n; i += TOPK_THREADS) {
-            unsigned key = order_key(row[i]);
-            if ((key & himask) == prefix) atomicAdd(&hist[(key >> shift) & 0xffu], 1u);
-        }
-        __syncthreads();
-        if (warp == 0) {
-            // the bin where the count from the top reaches `need` (bin 0 if it never does before it):
-            // lane L sums bins 255 - 8L .. 248 - 8L, a warp scan finds the lane, the lane walks its 8 bins
-            const unsigned need = s_need;
-            unsigned c[8], tot = 0;
-#pragma unroll
-            for (int j = 0; j < 8; j++) { c[j] = hist[255 - 8 * lane - j]; tot += c[j]; }
-            unsigned inc = tot;
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const unsigned v = __shfl_up_sync(0xffffffffu, inc, off);
-                if (lane >= off) inc += v;
-            }
-            const unsigned exc = inc - tot;
-            const unsigned hit = __ballot_sync(0xffffffffu, exc < need && inc >= need);
-            const int owner = hit ? __ffs(hit) - 1 : 31;
-            if (lane == owner) {
-                unsigned acc = exc;
-                int b = 0;
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const int bin = 255 - 8 * lane - j;
-                    if (bin == 0) break;                          // bin 0 takes whatever is left
-                    if (acc + c[j] >= need) { b = bin; break; }
-                    acc += c[j];
-                }
-                s_greater += acc;
-                s_need = need - acc;
-                s_prefix = prefix | ((unsigned)b << shift);
-            }
-        }
-        __syncthreads();
-    }
-    const unsigned T = s_prefix;
-    const unsigned n_greater = s_greater;          // scores with key > T
-    const unsigned n_ties = (unsigned)k - n_greater;   // lowest-index scores == T to take
-    if (tid == 0) { s_taken = 0; s_base = 0; }
-    __syncthreads();
-
-    // index-ordered sweep: greater keys go to slots [0, n_greater) in any order
-    // (sorted below); ties are appended in ascending index order.
-    __shared__ unsigned w_tie[TOPK_THREADS / 32];
-    for (int base = 0; base < n; base += TOPK_THREADS) {
-        int i = base + tid;
-        unsigned key = i < n ? order_key(row[i]) : 0u;
-        bool gt = i < n && key > T;
-        bool eq = i < n && key == T;
-        if (gt) {
-            unsigned slot = atomicAdd(&s_taken, 1u);
-            sel[slot] = ((unsigned long long)key << 32) | (0xffffffffu - (unsigned)i);
-        }
-        unsigned m = __ballot_sync(0xffffffffu, eq);
-        if (lane == 0) w_tie[warp] = __popc(m);
-        __syncthreads();
-        unsigned before = 0;
-        for (int w = 0; w < warp; w++) before += w_tie[w];
-        unsigned total = 0;
-        for (int w = 0; w < TOPK_THREADS / 32; w++) total += w_tie[w];
-        unsigned rank = s_base + before + __popc(m & ((1u << lane) - 1u));
-        if (eq && rank < n_ties)
-            sel[n_greater + rank] = ((unsigned long long)key << 32) | (0xffffffffu - (unsigned)i);
-        __syncthreads();
-        if (tid == 0) s_base += total;
-        __syncthreads();
-    }
-    }
-
-    // bitonic sort, descending, on the composite (key, -index)
-    int kp = 1;
-    while (kp < k) kp <<= 1;
-    for (int i = k + tid; i < kp; i += TOPK_THREADS) sel[i] = 0ull;
-    __syncthreads();
-    for (int size = 2; size <= kp; size <<= 1)
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int i = tid; i < kp; i += TOPK_THREADS) {
-                int j = i ^ stride;
-                if (j > i) {
-                    unsigned long long a = sel[i], b = sel[j];
-                    bool desc = ((i & size) == 0);
-                    if (desc ? (a < b) : (a > b)) { sel[i] = b; sel[j] = a; }
-                }
-            }
-            __syncthreads();
-        }
-    for (int i = tid; i < k; i += TOPK_THREADS)
-        out[i] = (int32_t)(0xffffffffu - (unsigned)(sel[i] & 0xffffffffu));
-}
-
-// The same selection for long rows, a row spread over a cluster of TOPK_CL CTAs (one CTA sweeping 262,144
-// scores five times takes ~350 us): every CTA histograms its slice, all of them add the eight histograms
-// through distributed shared memory and derive the same digit, so no result has to be sent around; the
-// chosen entries are stored into rank 0's shared memory (greater keys at slots counted per slice, ties in
-// index order behind them), where rank 0 sorts and writes them out.  Nobody touches another CTA's shared
-// memory before a first cluster barrier (a CTA of the cluster may not have started yet), and nobody leaves
-// before the last reader is done.
-#define TOPK_CL 8
-__global__ void __cluster_dims__(TOPK_CL, 1, 1) __launch_bounds__(TOPK_THREADS)
-topk_stable_cl_kernel(const float *__restrict__ scores, int n, int k, int32_t *__restrict__ idx_out,
-                      const long long *__restrict__ dyn_pos, int ratio, long long chunk_pos0, int rows_per_pos) {
     namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
-    __shared__ unsigned hist[256];
-    __shared__ unsigned ghist[2][256];                 // rank 0's copies: the eight slices' histograms added up
-    __shared__ unsigned s_digit[2];
-    __shared__ unsigned s_cnt[2];                      // this slice's keys > T and keys == T
-    __shared__ unsigned s_taken, s_base;
-    __shared__ unsigned w_tie[TOPK_THREADS / 32];
-    __shared__ unsigned long long sel[TOPK_MAX_K];     // rank 0's copy collects the choice
-    const int rowi = blockIdx.x / TOPK_CL, rank = (int)cluster.block_rank();
+    __shared__ unsigned hist[TOPK_BINS];
+    __shared__ unsigned ghist[CL > 1 ? 2 : 1][CL > 1 ? TOPK_BINS : 1];   // rank 0's copies: the slices' histograms added up
+    __shared__ unsigned s_w[32], s_digit[3];
+    __shared__ unsigned s_eq;                           // this slice's keys equal to the boundary
+    __shared__ unsigned s_taken;                        // rank 0's copy counts the chosen entries
+    __shared__ unsigned long long sel[TOPK_MAX_K];      // rank 0's copy collects the choice
+    const int rowi = blockIdx.x / CL, rank = CL > 1 ? (int)(blockIdx.x % CL) : 0;
     const float *row = scores + (size_t)rowi * n;       // n, k as given are the row strides
     int32_t *out = idx_out + (size_t)rowi * k;
-    if (dyn_pos || rows_per_pos > 0) {
+    if (dyn_pos || rows_per_pos > 0) {                  // live sizes from the position (of the row, in a chunk)
         const long long nbs = ((dyn_pos ? *dyn_pos : chunk_pos0 + rowi / rows_per_pos) + 1) / ratio;
         n = (int)(nbs < n ? nbs : n);
         k = k < n ? k : n;
     }
-    cluster.sync();                                    // every CTA of the cluster runs from here on
-    if (k <= 0) return;                                // the same decision in all eight
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int per = (n + TOPK_CL - 1) / TOPK_CL, i0 = min(n, rank * per), i1 = min(n, i0 + per);
-    unsigned prefix = 0, need = (unsigned)(k < n ? k : n), n_greater = 0;
-    const bool all = k >= n;                           // every score is taken: only the order is left
-    if (all) k = n;
-    unsigned *g0 = cluster.map_shared_rank(&ghist[0][0], 0);     // rank 0 holds the summed histograms (two, alternating)
-    for (int pass = 0; pass < 4 && !all; pass++) {
-        const int shift = 24 - 8 * pass;
-        unsigned *gh = g0 + (pass & 1) * 256;
-        for (int i = tid; i < 256; i += TOPK_THREADS) {
+    auto sync_all = [&]() { if constexpr (CL > 1) cg::this_cluster().sync(); else __syncthreads(); };
+    auto at_rank = [&](unsigned *p, int r) -> unsigned * {
+        if constexpr (CL > 1) return cg::this_cluster().map_shared_rank(p, r);
+        else return p;
+    };
+    if (tid == 0) { s_taken = 0; s_eq = 0; }
+    sync_all();                                         // every CTA of the cluster runs from here on
+    if (k <= 0) return;                                 // the same decision in all of them
+    const int per = (n + CL - 1) / CL, i0 = min(n, rank * per), i1 = min(n, i0 + per);
+    const int steps = (per + TOPK_THREADS - 1) / TOPK_THREADS;       // the same in every CTA
+    uint32_t keys[KPT ? KPT : 1];
+    if (KPT) {
+#pragma unroll
+        for (int r = 0; r < KPT; r++) {
+            const int i = i0 + r * TOPK_THREADS + tid;
+            keys[r] = i < i1 ? order_key(row[i]) : 0u;
+        }
+    }
+    // calls f(i, key) for this thread's scores in ascending order; whole warps stay together (in = a real score)
+    auto each = [&](auto &&f) {
+        if constexpr (KPT > 0) {
+#pragma unroll
+            for (int r = 0; r < KPT; r++) {
+                if (r >= steps) break;
+                const int i = i0 + r * TOPK_THREADS + tid;
+                f(i, keys[r], i < i1);
+            }
+        } else {
+            for (int r = 0; r < steps; r++) {
+                const int i = i0 + r * TOPK_THREADS + tid;
+                f(i, i < i1 ? order_key(row[i]) : 0u, i < i1);
+            }
+        }
+    };
+    uint32_t T = 0;                                     // boundary so far: the digits of the k-th key, zeros below
+    unsigned need = (unsigned)k, n_greater = 0;         // of the keys that share its digits; keys above them
+    bool whole = k >= n;                                // every key >= T is chosen
+    if (k > n) k = n;
+    for (int pass = 0; pass < 3 && !whole; pass++) {
+        const int shift = pass == 0 ? 21 : pass == 1 ? 10 : 0;
+        const uint32_t himask = pass == 0 ? 0u : pass == 1 ? 0xffe00000u : 0xfffffc00u, dmask = pass == 2 ? 1023u : 2047u;
+        for (int i = tid; i < TOPK_BINS; i += TOPK_THREADS) {
             hist[i] = 0;
-            if (rank == 0) ghist[pass & 1][i] = 0;             // last read two barriers ago
+            if (CL > 1 && rank == 0) ghist[pass & 1][i] = 0;         // last read two barriers ago
         }
-        cluster.sync();
-        const unsigned himask = pass ? (0xffffffffu << (shift + 8)) : 0u;
-        for (int i = i0 + tid; i < i1; i += TOPK_THREADS) {
-            const unsigned key = order_key(row[i]);
-            if ((key & himask) == prefix) atomicAdd(&hist[(key >> shift) & 0xffu], 1u);
-        }
+        sync_all();
+        each([&](int, uint32_t key, bool in) {
+            if (in && (key & himask) == T) atomicAdd(&hist[(key >> shift) & dmask], 1u);
+        });
         __syncthreads();
-        if (tid < 256 && hist[tid]) atomicAdd(gh + tid, hist[tid]);   // one remote add per bin and CTA
-        cluster.sync();                                // the sum is complete
-        if (warp == 0) {
-            // the digit from the summed histogram (lane L: bins 255-8L .. 248-8L), the same in every CTA
-            unsigned c[8], tot = 0;
+        const unsigned *h = hist;
+        if (CL > 1) {
+            unsigned *g = at_rank(&ghist[pass & 1][0], 0);
+            for (int i = tid; i < TOPK_BINS; i += TOPK_THREADS)
+                if (hist[i]) atomicAdd(g + i, hist[i]);
+            sync_all();                                 // the sum is complete
+            h = g;
+        }
+        // the bin where the count from the top reaches `need`: thread t holds bins 2047 - 2t and 2046 - 2t
+        const unsigned c0 = h[TOPK_BINS - 1 - 2 * tid], c1 = h[TOPK_BINS - 2 - 2 * tid], tot = c0 + c1;
+        unsigned inc = tot;
 #pragma unroll
-            for (int j = 0; j < 8; j++) { c[j] = gh[255 - 8 * lane - j]; tot += c[j]; }
-            unsigned inc = tot;
+        for (int off = 1; off < 32; off <<= 1) {
+            const unsigned v = __shfl_up_sync(0xffffffffu, inc, off);
+            if (lane >= off) inc += v;
+        }
+        if (lane == 31) s_w[warp] = inc;
+        __syncthreads();
+        unsigned wv = s_w[lane];
 #pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const unsigned v = __shfl_up_sync(0xffffffffu, inc, off);
-                if (lane >= off) inc += v;
-            }
-            const unsigned exc = inc - tot;
-            const unsigned hit = __ballot_sync(0xffffffffu, exc < need && inc >= need);
-            const int owner = hit ? __ffs(hit) - 1 : 31;
-            if (lane == owner) {
-                unsigned acc = exc;
-                int b = 0;
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const int bin = 255 - 8 * lane - j;
-                    if (bin == 0) break;                    // bin 0 takes whatever is left
-                    if (acc + c[j] >= need) { b = bin; break; }
-                    acc += c[j];
-                }
-                s_digit[0] = acc; s_digit[1] = (unsigned)b;
-            }
+        for (int off = 1; off < 32; off <<= 1) {
+            const unsigned v = __shfl_up_sync(0xffffffffu, wv, off);
+            if (lane >= off) wv += v;
+        }
+        const unsigned before = warp ? __shfl_sync(0xffffffffu, wv, (warp + 31) & 31) : 0u;
+        const unsigned exc = before + inc - tot;
+        if (exc < need && exc + tot >= need) {          // one thread: the counts add up to at least `need`
+            const bool first = exc + c0 >= need;
+            s_digit[0] = first ? exc : exc + c0;
+            s_digit[1] = (unsigned)(first ? TOPK_BINS - 1 - 2 * tid : TOPK_BINS - 2 - 2 * tid);
+            s_digit[2] = first ? c0 : c1;
         }
         __syncthreads();
         n_greater += s_digit[0];
         need -= s_digit[0];
-        prefix |= s_digit[1] << shift;
-        __syncthreads();                               // s_digit is rewritten in the next pass
+        T |= s_digit[1] << shift;
+        whole = s_digit[2] == need;
     }
-    const unsigned T = all ? 0u : prefix;
-    const unsigned n_ties = all ? 0u : (unsigned)k - n_greater;
-    // this slice's counts, then where its entries go: greater keys after those of lower slices, ties (in
-    // index order) after the ties of lower slices
-    if (tid == 0) { s_cnt[0] = 0; s_cnt[1] = 0; s_taken = 0; s_base = 0; }
-    __syncthreads();
-    {
-        unsigned g = 0, e = 0;
-        for (int i = i0 + tid; i < i1; i += TOPK_THREADS) {
-            const unsigned key = order_key(row[i]);
-            g += all || key > T;
-            e += !all && key == T;
-        }
-        g = __reduce_add_sync(0xffffffffu, g);
-        e = __reduce_add_sync(0xffffffffu, e);
-        if (lane == 0) { atomicAdd(&s_cnt[0], g); atomicAdd(&s_cnt[1], e); }
+    // keys above the boundary (all those at it too, when they are all chosen) in any order
+    unsigned *cnt0 = at_rank(&s_taken, 0);
+    unsigned long long *sel0 = sel;
+    if constexpr (CL > 1) sel0 = cg::this_cluster().map_shared_rank(sel, 0);
+    unsigned eq = 0;
+    each([&](int i, uint32_t key, bool in) {
+        const bool take = in && (whole ? key >= T : key > T);
+        eq += !whole && in && key == T;
+        const unsigned m = __ballot_sync(0xffffffffu, take);
+        if (!m) return;
+        unsigned slot = 0;
+        if (lane == 0) slot = atomicAdd(cnt0, (unsigned)__popc(m));
+        slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(m & ((1u << lane) - 1u));
+        if (take) sel0[slot] = ((unsigned long long)key << 32) | (0xffffffffu - (unsigned)i);
+    });
+    if (!whole) {
+        // more keys at the boundary than places: the lowest indices, counted over the slices before this one
+        // and, inside the slice, step by step
+        eq = __reduce_add_sync(0xffffffffu, eq);
+        if (lane == 0 && eq) atomicAdd(&s_eq, eq);
+        sync_all();
+        unsigned base = 0;
+        for (int q = 0; q < rank; q++) base += *at_rank(&s_eq, q);
+        each([&](int i, uint32_t key, bool in) {
+            const bool e = in && key == T;
+            const unsigned m = __ballot_sync(0xffffffffu, e);
+            if (lane == 0) s_w[warp] = __popc(m);
+            __syncthreads();
+            unsigned wv = s_w[lane], tot = __reduce_add_sync(0xffffffffu, wv);
+            const unsigned bef = __reduce_add_sync(0xffffffffu, lane < warp ? wv : 0u);
+            const unsigned place = base + bef + __popc(m & ((1u << lane) - 1u));
+            if (e && place < need) sel0[n_greater + place] = ((unsigned long long)key << 32) | (0xffffffffu - (unsigned)i);
+            base += tot;
+            __syncthreads();
+        });
     }
-    cluster.sync();
-    unsigned g_base = 0, e_base = 0;
-    for (int q = 0; q < rank; q++) {
-        const unsigned *cq = cluster.map_shared_rank(s_cnt, q);
-        g_base += cq[0]; e_base += cq[1];
-    }
-    unsigned long long *sel0 = cluster.map_shared_rank(sel, 0);
-    for (int base = i0; base < i1; base += TOPK_THREADS) {
-        const int i = base + tid;
-        const unsigned key = i < i1 ? order_key(row[i]) : 0u;
-        const bool gt = i < i1 && (all || key > T);
-        const bool eq = i < i1 && !all && key == T;
-        if (gt) {
-            const unsigned slot = g_base + atomicAdd(&s_taken, 1u);
-            sel0[slot] = ((unsigned long long)key << 32) | (0xffffffffu - (unsigned)i);
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, eq);
-        if (lane == 0) w_tie[warp] = __popc(m);
-        __syncthreads();
-        unsigned before = 0, total = 0;
-        for (int w = 0; w < TOPK_THREADS / 32; w++) {
-            if (w < warp) before += w_tie[w];
-            total += w_tie[w];
-        }
-        const unsigned trank = e_base + s_base + before + __popc(m & ((1u << lane) - 1u));
-        if (eq && trank < n_ties)
-            sel0[n_greater + trank] = ((unsigned long long)key << 32) | (0xffffffffu - (unsigned)i);
-        __syncthreads();
-        if (tid == 0) s_base += total;
-        __syncthreads();
-    }
-    cluster.sync();                                    // the whole choice sits in rank 0
+    sync_all();                                         // the whole choice sits in rank 0
     if (rank != 0) return;
-    int kp = 1;
+    // bitonic sort, descending, on the composite (key, -index)
+    int kp = 32;
     while (kp < k) kp <<= 1;
+    if (kp <= TOPK_THREADS) {
+        unsigned long long v = tid < k ? sel[tid] : 0ull;
+        int buf = 0;
+        __syncthreads();
+        for (int size = 2; size <= kp; size <<= 1)
+            for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                unsigned long long w;
+                if (stride >= 32) {                     // the two halves of `sel` in turn: one barrier per exchange
+                    if (tid < kp) sel[buf * TOPK_THREADS + tid] = v;
+                    __syncthreads();
+                    w = tid < kp ? sel[buf * TOPK_THREADS + (tid ^ stride)] : 0ull;
+                    buf ^= 1;
+                } else {
+                    w = __shfl_xor_sync(0xffffffffu, v, stride);
+                }
+                const bool want_max = ((tid & size) == 0) == ((tid & stride) == 0);
+                v = want_max == (v > w) ? v : w;
+            }
+        if (tid < k) out[tid] = (int32_t)(0xffffffffu - (unsigned)(v & 0xffffffffu));
+        return;
+    }
     for (int i = k + tid; i < kp; i += TOPK_THREADS) sel[i] = 0ull;
     __syncthreads();
     for (int size = 2; size <= kp; size <<= 1)
@@ -313,12 +237,19 @@ int topk_stable(const float *scores, int n, int k, int32_t *idx, int rows,
     APUS_REQUIRE(k >= 1 && (k <= n || dyn_pos || rows_per_pos > 0) && k <= TOPK_MAX_K, "topk: n=%d k=%d unsupported", n, k);
     if (rows <= 0) return 0;
     static const int cl_min = [] { const char *e = getenv("APUS_TOPK_CLUSTER_MIN"); return e && e[0] ? atoi(e) : 16384; }();
+#define TOPK_LAUNCH(CL, KPT)                                                                                              \
+    launch_k(topk_stable_kernel<CL, KPT>, (unsigned)rows * CL, TOPK_THREADS, 0, st, scores, n, k, idx, dyn_pos, ratio,    \
+             chunk_pos0, rows_per_pos)
     if (n >= cl_min) {                                  // long rows: a cluster of CTAs per row
-        topk_stable_cl_kernel<<<rows * TOPK_CL, TOPK_THREADS, 0, st>>>(scores, n, k, idx, dyn_pos, ratio, chunk_pos0, rows_per_pos);
-        APUS_LAUNCHED();
-        return 0;
+        if (n <= TOPK_CL * TOPK_THREADS * 8) TOPK_LAUNCH(TOPK_CL, 8);
+        else if (n <= TOPK_CL * TOPK_THREADS * 32) TOPK_LAUNCH(TOPK_CL, 32);
+        else TOPK_LAUNCH(TOPK_CL, 0);
+    } else {
+        if (n <= TOPK_THREADS * 4) TOPK_LAUNCH(1, 4);
+        else if (n <= TOPK_THREADS * 16) TOPK_LAUNCH(1, 16);
+        else TOPK_LAUNCH(1, 0);
     }
-    launch_k(topk_stable_kernel, rows, TOPK_THREADS, 0, st, scores, n, k, idx, dyn_pos, ratio, chunk_pos0, rows_per_pos);
+#undef TOPK_LAUNCH
     APUS_LAUNCHED();
     return 0;
 }

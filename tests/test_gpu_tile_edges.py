@@ -3,7 +3,8 @@ kernel of this library that knows no tiles."""
 import numpy as np
 import pytest
 
-from _gpu import bits, cuda_moe, cuda_qgemm
+from _gpu import bits, cuda_moe, cuda_qgemm, lib
+from _oracle import P
 from apus_b200 import synth
 
 pytestmark = pytest.mark.gpu
@@ -37,3 +38,29 @@ def test_grouping_of_many_routings(T):
         part = cuda_moe(W, x[lo:lo + 7])
         assert np.array_equal(whole["idx"][lo:lo + 7], part["idx"])
         assert np.array_equal(bits(whole["out"][lo:lo + 7]), bits(part["out"]))
+
+
+@pytest.mark.parametrize("n,k", [(1, 1), (31, 31), (33, 7), (1024, 512), (2049, 512), (4097, 2048), (5000, 1), (16383, 1025), (16384, 512),
+                                 (65537, 512), (70001, 2048), (262144, 512), (262147, 40)])
+@pytest.mark.parametrize("values", ["normal", "coarse", "one", "ends"])
+def test_topk_selection(n, k, values):
+    """Every layout of the selection (keys in registers or read again, one CTA or a cluster): order by (score
+    descending, index ascending), with ties at the boundary, one value everywhere, infinities and both zeros."""
+    rng = np.random.default_rng(n + k)
+    rows = 3
+    sc = rng.standard_normal((rows, n)).astype(np.float32)
+    if values == "coarse":
+        sc = synth.bf16_round(sc)
+        sc[1] = np.round(sc[1])
+    elif values == "one":
+        sc[:] = np.float32(-0.25)
+        sc[1, n // 2] = 3.0
+    elif values == "ends":
+        sc[:, rng.integers(0, n, 3)] = np.inf
+        sc[:, rng.integers(0, n, 3)] = -np.inf
+        sc[1] = np.where(rng.random(n) < 0.5, np.float32(0.0), np.float32(-0.0))
+        sc[2] = np.finfo(np.float32).min
+    idx = np.empty((rows, k), np.int32)
+    assert lib().apus_cuda_topk_stable(P(sc), n, k, P(idx), rows) == 0, lib().apus_cuda_last_error()
+    want = np.argsort(-(sc + np.float32(0)).astype(np.float64), axis=1, kind="stable")[:, :k]
+    assert np.array_equal(idx, want)

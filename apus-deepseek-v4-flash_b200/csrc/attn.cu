@@ -3,6 +3,7 @@
 #include <cooperative_groups.h>
 #include "common.cuh"
 #include "kernels.cuh"
+#include "tc_common.cuh"
 
 namespace apus {
 
@@ -400,176 +401,269 @@ sparse_pv_kernel(const float *__restrict__ sc, const float *__restrict__ sink, i
 }
 
 // ---- the same two steps, register-tiled ---------------------------------------------------------
-// Same arithmetic, same order, same bits as the two kernels above; what changes is how often a
-// number is fetched per flop.
+// Same arithmetic, same order, same bits as the two kernels above; what changes is how often a number is
+// fetched per flop and how many instructions a flop takes.
 //
-// Scores: a warp owns a tile of 16 heads x 32 candidates and walks k in chunks of 64 staged in shared
-// memory TRANSPOSED (q chunk [k][16 heads], KV chunk [k][32 ids], pitch 36 words so the 16-byte
-// stores of four gathered rows at one k do not collide); a lane owns 4 heads x 4 candidates, so one
-// k costs it two 16-byte shared loads for 16 multiply-add pairs -- the kernel is bound by the FP32
-// pipes (its floor: every (head, candidate) dot is 512 dependent multiply/add pairs), where the
-// kernel above is bound by shared-memory loads at one 4-byte load per flop.
+// Both contractions are chains of (multiply, add) per (head, candidate) or (head, channel), bound by the
+// FP32 pipes.  Two things shorten them without touching a bit:
+//   - q, the KV rows and the probabilities are BF16 values, so a product is exact and one fused
+//     multiply-add returns what the multiply and the add return.  That holds inside an exponent window
+//     (fma_ok_f32); every operand is examined, and where one lies outside (or is a true f32 value) the
+//     two-instruction walk runs instead.  What the scores kernel and the softmax find about the rows and the
+//     probabilities of a token is left in bad[t] for P.V.
+//   - two accumulators per instruction (f32x2): two heads in the scores, two channels in P.V.
+// One packed instruction does two multiply-adds at the rate of two scalar ones, in half the issue slots; the kernels
+// still spend as many on operand moves, and the FP32 pipes are 30-45 % busy.  Times beside the launches below.
+//
+// Scores: a lane owns HL heads x CL candidates, a warp 4 HL heads x 8 CL candidates, a CTA WH x WC warps.
+// The CTA's gathered rows travel 128 bytes of k at a time, three chunks deep, in their natural layout by
+// 16-byte cp.async (row pitch 36 words: the eight rows the lanes of a load touch fall into different banks);
+// the q chunk sits transposed ([k][head], a 16-byte load gives a lane two head pairs), its 4-head groups
+// permuted by k so that the transposing stores do not collide, and passes through registers: loaded before
+// the arithmetic of a chunk, stored after it.
 // softmax: max, p_j = bf16(exp(s_j - max)) written over the scores, denominator per (row, head).
-// P.V: a CTA owns HG heads of a row; a thread owns one channel pair for all HG heads (accumulators
-// in registers), so a gathered KV row is fetched once per HG heads instead of once per head; the
-// probabilities of a chunk of candidates sit transposed in shared memory ([j][HG], one 16-byte
-// broadcast load per 4 heads).
 #define SS_ROWB 128                       // bytes of a KV row staged per chunk: 64 BF16 or 32 f32 values of k
 #define SS_PITCHW 36                      // row pitch of the staged tile in 32-bit words (128 B + 16 B pad)
+#define SS_NS 3
 
-// Scores.  A warp owns 16 heads x 8 NB candidates; lane = (hg, jg) owns heads 4hg..4hg+3 and candidates
-// jg, jg+8, ... (NB of them: 4 where the launch fills the GPU anyway; 1 for the few rows of a small step,
-// whose duration is one warp's instruction stream -- a quarter of it per warp and four times the warps).  The warp's 32 gathered rows are staged 128 bytes of k at a time in their
-// natural layout by 16-byte cp.async (two buffers: the next chunk is in flight while this one is
-// consumed); with a pitch of 36 words the eight rows the lanes of a load touch fall into different
-// banks.  The q chunk is shared by the CTA's warps, transposed ([k][16 heads]: one 16-byte load gives
-// a lane its four heads).  Per k a lane issues 5 shared loads for 16 multiply/add pairs.
-template <bool BF16, int W, int NB>
-__global__ void __launch_bounds__(32 * W)
+template <bool BF16, int HL, int CL, int WH, int WC>
+struct ScoreCfg {
+    static constexpr int THREADS = 32 * WH * WC, HEADS = 4 * HL * WH, CANDS = 8 * CL * WC, KC = BF16 ? 64 : 32;
+    static constexpr int Q_WORDS = KC * HEADS, STAGE = (Q_WORDS + CANDS * SS_PITCHW) * 4, SMEM = SS_NS * STAGE;
+};
+
+// The operands of four k for a lane: its head pairs and its candidates' words
+template <bool BF16, int HL, int CL, int HEADS>
+struct ScoreOps {
+    ulonglong2 q[4][HL / 4];
+    uint32_t kv[CL][BF16 ? 2 : 4];
+    __device__ __forceinline__ void load(const float *sq, const uint32_t *skv, int g0, int g) {
+        constexpr int SWZ = (HEADS / 4 < 8 ? HEADS / 4 : 8) - 1;
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+#pragma unroll
+            for (int i = 0; i < HL / 4; i++)
+                q[e][i] = *reinterpret_cast<const ulonglong2 *>(sq + (size_t)(4 * g + e) * HEADS + 4 * ((g0 + i) ^ (g & SWZ)));
+#pragma unroll
+        for (int b = 0; b < CL; b++) {
+            if constexpr (BF16) {
+                const uint2 r = *reinterpret_cast<const uint2 *>(skv + (size_t)8 * b * SS_PITCHW + 2 * g);
+                kv[b][0] = r.x; kv[b][1] = r.y;
+            } else {
+                const uint4 r = *reinterpret_cast<const uint4 *>(skv + (size_t)8 * b * SS_PITCHW + 4 * g);
+                kv[b][0] = r.x; kv[b][1] = r.y; kv[b][2] = r.z; kv[b][3] = r.w;
+            }
+        }
+    }
+    template <bool FUSED>
+    __device__ __forceinline__ void walk(f32x2 (&acc)[HL / 2][CL]) const {
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+#pragma unroll
+            for (int b = 0; b < CL; b++) {
+                const uint32_t u = BF16 ? (e & 1 ? kv[b][e >> 1] & 0xffff0000u : kv[b][e >> 1] << 16) : kv[b][BF16 ? 0 : e];
+                const f32x2 y = pack2(__uint_as_float(u), __uint_as_float(u));
+#pragma unroll
+                for (int a = 0; a < HL / 2; a++) acc[a][b] = mac2<FUSED>(acc[a][b], a & 1 ? q[e][a >> 1].y : q[e][a >> 1].x, y);
+            }
+    }
+};
+// One chunk of k for a lane, acc[pair of heads][candidate]; operands are read four k ahead of their use
+template <bool BF16, bool FUSED, int HL, int CL, int HEADS>
+__device__ __forceinline__ void score_chunk(f32x2 (&acc)[HL / 2][CL], const float *sq, const uint32_t *skv, int g0) {
+    constexpr int NG = (BF16 ? 64 : 32) / 4;
+    ScoreOps<BF16, HL, CL, HEADS> A, B;
+    A.load(sq, skv, g0, 0);
+#pragma unroll
+    for (int g = 0; g < NG; g += 2) {
+        B.load(sq, skv, g0, g + 1);
+        A.template walk<FUSED>(acc);
+        if (g + 2 < NG) A.load(sq, skv, g0, g + 2);
+        B.template walk<FUSED>(acc);
+    }
+}
+
+template <bool BF16, int HL, int CL, int WH, int WC>
+__global__ void __launch_bounds__(32 * WH * WC)
 sparse_scores_tile_kernel(const float *__restrict__ q, int h, int d, const int32_t *__restrict__ ids,
                           const int *__restrict__ ns, int idxw, float scale, const void *kv_a, int64_t na,
-                          const void *kv_b, float *__restrict__ sc, size_t a_stride, size_t b_stride, int seq_mod) {
+                          const void *kv_b, float *__restrict__ sc, size_t a_stride, size_t b_stride, int seq_mod,
+                          int *__restrict__ bad) {
     APUS_PDL_WAIT();
     APUS_PDL_GO();
-    constexpr int KC = BF16 ? 64 : 32;                         // k values per chunk
+    using Cf = ScoreCfg<BF16, HL, CL, WH, WC>;
+    constexpr int NT = Cf::THREADS, KC = Cf::KC, HEADS = Cf::HEADS, CANDS = Cf::CANDS;
+    constexpr int SWZ = (HEADS / 4 < 8 ? HEADS / 4 : 8) - 1;
     extern __shared__ __align__(16) unsigned char ss_raw[];
-    float (*s_q)[KC][16] = reinterpret_cast<float (*)[KC][16]>(ss_raw);                       // [2][KC][16]
-    constexpr int TJ = 8 * NB;                                  // candidates of a warp's tile
-    uint32_t (*s_kv)[2][TJ][SS_PITCHW] =
-        reinterpret_cast<uint32_t (*)[2][TJ][SS_PITCHW]>(ss_raw + 2 * KC * 16 * 4);           // [W][2][TJ][pitch]
-    const int t = blockIdx.z, hb = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int n = ns[t];
-    const int j0 = ((int)blockIdx.x * W + warp) * TJ;          // first candidate of this warp's tile
-    if ((int)blockIdx.x * W * TJ >= n) return;                  // whole CTA past the row
+    __shared__ int s_bad[SS_NS];                                // chunk in this stage: an operand outside the window
+    const int t = blockIdx.z, h0 = (int)blockIdx.y * HEADS, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int n = ns[t], j0 = (int)blockIdx.x * CANDS;
+    if (j0 >= n) return;                                        // whole CTA past the row
     const int own = seq_mod > 0 ? t % seq_mod : t;
     const size_t esz = BF16 ? 2 : 4;
-    // lane u-th copy of a chunk: row (lane + 32u) / 8, 16-byte segment (lane + 32u) % 8; the four rows a
-    // lane copies from are fixed, so their base pointers stay in registers
-    const char *rowp[2 * NB];
+    const int nchunk = d / KC;
+    // copy u of this thread: row (tid + NT u) / 8, 16-byte segment tid % 8; its rows are the same in every chunk
+    constexpr int NKV = (CANDS * 8 + NT - 1) / NT;
+    static_assert((CANDS * 8 % NT == 0 || NKV == 1) && NT % 8 == 0, "row copies must divide among the threads");
+    const bool copies = tid < CANDS * 8;                        // the smallest tile has fewer copies than threads
+    const char *rowp[NKV];
     const char *dummy = reinterpret_cast<const char *>(kv_a ? kv_a : kv_b);
 #pragma unroll
-    for (int u = 0; u < 2 * NB; u++) {
-        const int r = (lane + 32 * u) >> 3, j = j0 + r;
+    for (int u = 0; u < NKV; u++) {
+        const int j = j0 + ((tid + NT * u) >> 3);
         const char *ptr = nullptr;
-        if (j < n) {
+        if (copies && j < n) {
             const int32_t id = ids[(size_t)t * idxw + j];
             ptr = id < na ? reinterpret_cast<const char *>(kv_a) + (size_t)own * a_stride + (size_t)id * d * esz
                           : reinterpret_cast<const char *>(kv_b) + (size_t)own * b_stride + (size_t)(id - na) * d * esz;
+            ptr += (tid & 7) * 16;
         }
         rowp[u] = ptr;
     }
-    const bool live = j0 < n;                                   // warps past the row still help with the q chunk
-    const int hg = lane & 3, jg = lane >> 2;
-    const int nchunk = d / KC;
-    // the q chunk of the NEXT step travels through registers: loaded before this step's arithmetic,
-    // stored (transposed) after it, so its latency hides behind the multiply/adds
-    constexpr int QN = (KC * 16 + 32 * W - 1) / (32 * W);
-    float qreg[QN];
-    auto q_load = [&](int c) {
+    auto q_of = [&](int st) { return reinterpret_cast<float *>(ss_raw + (size_t)st * Cf::STAGE); };
+    auto kv_of = [&](int st) { return reinterpret_cast<uint32_t *>(ss_raw + (size_t)st * Cf::STAGE) + Cf::Q_WORDS; };
+    auto kv_stage = [&](int c) {
+        if (c < nchunk && copies) {
+            uint32_t *dst = kv_of(c % SS_NS);
 #pragma unroll
-        for (int u = 0; u < QN; u++) {
-            const int i = tid + 32 * W * u, hh = i / KC, kk = i - hh * KC, head = hb * 16 + hh;
-            qreg[u] = (i < KC * 16 && head < h) ? q[((size_t)t * h + head) * d + c * KC + kk] : 0.f;
-        }
-    };
-    auto q_store = [&](int buf) {
-#pragma unroll
-        for (int u = 0; u < QN; u++) {
-            const int i = tid + 32 * W * u, hh = i / KC, kk = i - hh * KC;
-            if (i < KC * 16) s_q[buf][kk][hh] = qreg[u];
-        }
-    };
-    auto kv_stage = [&](int c, int buf) {
-        if (live) {
-#pragma unroll
-            for (int u = 0; u < 2 * NB; u++) {
-                const int i = lane + 32 * u, r = i >> 3, seg = i & 7;
-                cp_async16(&s_kv[warp][buf][r][seg * 4], rowp[u] ? rowp[u] + (size_t)c * SS_ROWB + seg * 16 : dummy, rowp[u] != nullptr);
-            }
+            for (int u = 0; u < NKV; u++)
+                cp_async16(dst + (size_t)((tid + NT * u) >> 3) * SS_PITCHW + (tid & 7) * 4,
+                           rowp[u] ? rowp[u] + (size_t)c * SS_ROWB : dummy, rowp[u] != nullptr);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    float acc[4][NB];
+    constexpr int QN = HEADS * KC / 4 / NT;
+    static_assert(HEADS * (KC / 4) % NT == 0, "the q chunk must divide among the threads");
+    const bool q_vec = ((uintptr_t)q & 15) == 0;                // the caller's pointer may have any alignment
+    float4 qreg[QN];
+    auto q_load = [&](int c) {
 #pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < NB; b++) acc[a][b] = 0.f;
-    kv_stage(0, 0);
-    if (nchunk > 1) kv_stage(1, 1);
-    q_load(0);
-    q_store(0);
-    for (int c = 0; c < nchunk; c++) {
-        const int buf = c & 1;
-        if (c + 1 < nchunk) {
-            q_load(c + 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        for (int u = 0; u < QN; u++) {
+            const int i = tid + NT * u, hh = i / (KC / 4), seg = i % (KC / 4);
+            const float *src = q + ((size_t)t * h + h0 + hh) * d + c * KC + 4 * seg;
+            if (h0 + hh >= h) qreg[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            else if (q_vec) qreg[u] = *reinterpret_cast<const float4 *>(src);
+            else qreg[u] = make_float4(src[0], src[1], src[2], src[3]);
         }
-        __syncthreads();                                        // chunk c (q and the warp's rows) is visible
-        if (live) {
-            if (BF16) {
-#pragma unroll 4
-                for (int k2 = 0; k2 < KC / 2; k2++) {           // one 32-bit word holds k = 2 k2 and 2 k2 + 1
-                    const float4 qa = *reinterpret_cast<const float4 *>(&s_q[buf][2 * k2][4 * hg]);
-                    const float4 qb = *reinterpret_cast<const float4 *>(&s_q[buf][2 * k2 + 1][4 * hg]);
-                    const float q0[4] = {qa.x, qa.y, qa.z, qa.w}, q1[4] = {qb.x, qb.y, qb.z, qb.w};
-                    float k0v[NB], k1v[NB];
+    };
+    // stores chunk c's q and notes whether one of its values is outside the window
+    auto q_store = [&](int c) {
+        float *dst = q_of(c % SS_NS);
+        bool ok = true;
 #pragma unroll
-                    for (int b = 0; b < NB; b++) {
-                        const uint32_t w = s_kv[warp][buf][jg + 8 * b][k2];
-                        k0v[b] = __uint_as_float(w << 16);
-                        k1v[b] = __uint_as_float(w & 0xffff0000u);
-                    }
+        for (int u = 0; u < QN; u++) {
+            const int i = tid + NT * u, hh = i / (KC / 4), seg = i % (KC / 4);
+            float *p = dst + (size_t)4 * seg * HEADS + 4 * ((hh >> 2) ^ (seg & SWZ)) + (hh & 3);
+            p[0] = qreg[u].x; p[HEADS] = qreg[u].y; p[2 * HEADS] = qreg[u].z; p[3 * HEADS] = qreg[u].w;
+            ok = ok && fma_ok_f32(qreg[u].x) && fma_ok_f32(qreg[u].y) && fma_ok_f32(qreg[u].z) && fma_ok_f32(qreg[u].w);
+        }
+        if (!ok) s_bad[c % SS_NS] = 1;                          // every writer stores the same value
+    };
+    bool kv_bad = false;
+    // this thread's own copies of chunk c have landed: are they all in the window?
+    auto kv_check = [&](int c) {
+        if (!copies) return;
+        const uint32_t *src = kv_of(c % SS_NS);
+        uint32_t low = 0, mx = 0, mn = 0xffffffffu;             // f32 rows: low halves, largest and smallest non-zero |v|
 #pragma unroll
-                    for (int a = 0; a < 4; a++)
+        for (int u = 0; u < NKV; u++) {
+            const uint4 v = *reinterpret_cast<const uint4 *>(src + (size_t)((tid + NT * u) >> 3) * SS_PITCHW + (tid & 7) * 4);
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                        for (int b = 0; b < NB; b++) acc[a][b] = __fadd_rn(acc[a][b], __fmul_rn(q0[a], k0v[b]));
-#pragma unroll
-                    for (int a = 0; a < 4; a++)
-#pragma unroll
-                        for (int b = 0; b < NB; b++) acc[a][b] = __fadd_rn(acc[a][b], __fmul_rn(q1[a], k1v[b]));
-                }
-            } else {
-#pragma unroll 8
-                for (int kk = 0; kk < KC; kk++) {
-                    const float4 q4 = *reinterpret_cast<const float4 *>(&s_q[buf][kk][4 * hg]);
-                    const float qa[4] = {q4.x, q4.y, q4.z, q4.w};
-                    float kb[NB];
-#pragma unroll
-                    for (int b = 0; b < NB; b++) kb[b] = __uint_as_float(s_kv[warp][buf][jg + 8 * b][kk]);
-#pragma unroll
-                    for (int a = 0; a < 4; a++)
-#pragma unroll
-                        for (int b = 0; b < NB; b++) acc[a][b] = __fadd_rn(acc[a][b], __fmul_rn(qa[a], kb[b]));
-                }
+            for (int e = 0; e < 4; e++) {
+                if (BF16) low |= fma_bad_bf16x2(w[e]);
+                else { low |= w[e]; mx = max(mx, w[e] << 1); mn = min(mn, (w[e] << 1) - 1u); }
             }
         }
-        if (c + 1 < nchunk) q_store(buf ^ 1);                   // read last at step c - 1, behind that step's barrier
-        __syncthreads();                                        // this step's buffers are free again
-        if (c + 2 < nchunk) kv_stage(c + 2, buf);
+        const bool ok = BF16 ? (low & 0x80008000u) == 0u : (low & 0xffffu) == 0u && mx < (187u << 24) && mn >= (67u << 24) - 1u;
+        if (!ok) { s_bad[c % SS_NS] = 1; kv_bad = true; }
+    };
+    const int wh = warp % WH, wc = warp / WH, hg = lane & 3, jg = lane >> 2;
+    const bool live = j0 + wc * 8 * CL < n && h0 + wh * 4 * HL < h;     // other warps only help with the staging
+    f32x2 acc[HL / 2][CL];
+#pragma unroll
+    for (int a = 0; a < HL / 2; a++)
+#pragma unroll
+        for (int b = 0; b < CL; b++) acc[a][b] = 0ull;
+    if (tid < SS_NS) s_bad[tid] = 0;
+    kv_stage(0);
+    kv_stage(1);
+    q_load(0);
+    __syncthreads();                                            // the flags are clear
+    q_store(0);
+    for (int c = 0; c < nchunk; c++) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");    // the newest group is chunk c + 1
+        kv_check(c);
+        __syncthreads();                                        // chunk c is visible; chunk c - 1 has been consumed
+        kv_stage(c + 2);
+        if (c + 1 < nchunk) q_load(c + 1);
+        const bool fused = s_bad[c % SS_NS] == 0;
+        if (tid == 0) s_bad[(c + 2) % SS_NS] = 0;               // read last at chunk c - 1, written next for chunk c + 2
+        if (live) {
+            const float *sq = q_of(c % SS_NS);
+            const uint32_t *skv = kv_of(c % SS_NS) + (size_t)(wc * 8 * CL + jg) * SS_PITCHW;
+            const int g0 = (wh * 4 + hg) * (HL / 4);
+            if (fused) score_chunk<BF16, true, HL, CL, HEADS>(acc, sq, skv, g0);
+            else score_chunk<BF16, false, HL, CL, HEADS>(acc, sq, skv, g0);
+        }
+        if (c + 1 < nchunk) q_store(c + 1);                     // this stage was consumed at chunk c - 2
     }
+    if (kv_bad) bad[t] = 1;
     if (!live) return;
 #pragma unroll
-    for (int a = 0; a < 4; a++) {
-        const int head = hb * 16 + 4 * hg + a;
-        if (head >= h) continue;
+    for (int a = 0; a < HL / 2; a++) {
+        const int head = h0 + (wh * 4 + hg) * HL + 2 * a;
 #pragma unroll
-        for (int b = 0; b < NB; b++) {
-            const int j = j0 + jg + 8 * b;
-            if (j < n) sc[((size_t)t * h + head) * idxw + j] = __fmul_rn(acc[a][b], scale);
+        for (int b = 0; b < CL; b++) {
+            const int j = j0 + wc * 8 * CL + jg + 8 * b;
+            const float2 v = unpack2(acc[a][b]);
+            if (j < n && head < h) sc[((size_t)t * h + head) * idxw + j] = __fmul_rn(v.x, scale);
+            if (j < n && head + 1 < h) sc[((size_t)t * h + head + 1) * idxw + j] = __fmul_rn(v.y, scale);
         }
     }
+}
+
+// The same for rows of at most 1024 candidates, a warp per (row, head): the denominator is one lane's chain of n adds,
+// and eight of them run side by side in a CTA instead of one with seven idle warps beside it.
+// B200: 2,048 rows x 64 heads, up to 256 candidates 344 -> 134 us.
+__global__ void __launch_bounds__(256)
+sparse_softmax_rows_kernel(float *__restrict__ sc, const float *__restrict__ sink, int h, const int *__restrict__ ns, int idxw,
+                           float *__restrict__ den, int *__restrict__ bad) {
+    APUS_PDL_WAIT();
+    APUS_PDL_GO();
+    extern __shared__ __align__(16) float s_all[];           // [8][pitch]
+    const int t = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, head = (int)blockIdx.x * 8 + warp;
+    const int n = ns[t];
+    if (n == 0 || head >= h) return;
+    float *s_p = s_all + (size_t)warp * ((idxw + 3) & ~3);
+    float *sr = sc + ((size_t)t * h + head) * idxw;
+    float mx = -INFINITY;
+    for (int j = lane; j < n; j += 32) {
+        const float v = sr[j];
+        s_p[j] = v;
+        mx = fmaxf(mx, v);
+    }
+    mx = warp_max(mx);
+    bool ok = true;
+    for (int j = lane; j < n; j += 32) {
+        const float p = bf16_round(exp_rn(__fsub_rn(s_p[j], mx)));
+        s_p[j] = p;
+        sr[j] = p;
+        ok = ok && fma_ok_f32(p);
+    }
+    if (!ok) bad[t] = 1;                       // P.V takes the two-instruction walk
+    __syncwarp();
+    if (lane == 0) den[(size_t)t * h + head] = __fadd_rn(seq_sum_smem(s_p, n, 0.f), exp_rn(__fsub_rn(sink[head], mx)));
 }
 
 // max, p over the scores, the denominator sum_j p_j + exp(sink - max): the sums in the order of
 // sparse_pv_kernel (one accumulator for n <= 1024, the strided tree above it)
 __global__ void __launch_bounds__(256)
 sparse_softmax_kernel(float *__restrict__ sc, const float *__restrict__ sink, int h, const int *__restrict__ ns, int idxw,
-                      float *__restrict__ den) {
+                      float *__restrict__ den, int *__restrict__ bad) {
     APUS_PDL_WAIT();
     APUS_PDL_GO();
-    extern __shared__ float s_p[];             // [idxw]
+    extern __shared__ __align__(16) float s_p[];             // [idxw]
     __shared__ float red[32];
     __shared__ float s_mx, s_sum;
     const int t = blockIdx.y, head = blockIdx.x, tid = threadIdx.x;
@@ -592,13 +686,10 @@ sparse_softmax_kernel(float *__restrict__ sc, const float *__restrict__ sink, in
         const float p = bf16_round(exp_rn(__fsub_rn(sr[j], mx)));
         s_p[j] = p;
         sr[j] = p;
+        if (!fma_ok_f32(p)) bad[t] = 1;        // P.V takes the two-instruction walk
     }
     __syncthreads();
-    if (tid == 0 && n <= 1024) {
-        float sum = 0.f;
-        for (int j = 0; j < n; j++) sum = __fadd_rn(sum, s_p[j]);
-        s_sum = sum;
-    }
+    if (tid == 0 && n <= 1024) s_sum = seq_sum_smem(s_p, n, 0.f);
     if (n > 1024) {                            // long rows: tree sum
         float part = 0.f;
         for (int j = tid; j < n; j += blockDim.x) part += s_p[j];
@@ -704,120 +795,229 @@ sparse_pv_tile_kernel(const float *__restrict__ p, const float *__restrict__ den
     }
 }
 
-// P.V for the few (row, head group)s of a small step.  There the kernel above is a chain of load latencies:
-// a thread fetches a batch of gathered rows into registers, waits, accumulates, fetches the next -- and one
-// or two warps per SM keep too few bytes in flight to pull the rows out of L2 any faster.  Here a CTA owns
-// 4 heads x PVS_NP channel pairs of a row and stages the row segments of PVS_T candidates at a time in
-// shared memory with 16-byte asynchronous copies, two tiles in flight while a third is consumed (the
-// probabilities travel the same way, 4 bytes each), so the copies of the whole row are issued back to
-// back and the accumulation reads shared memory.  Same products, same order of adds, same bits.
+// P.V from staged rows.  A CTA owns HG heads x 2 NPAIR NT channels of a row; a thread owns NPAIR channel pairs
+// for all HG heads (one f32x2 accumulator each).  The row segments of T candidates at a time come in two tiles ahead
+// of the one that is consumed, by 16-byte cp.async or (BULK) by one bulk copy per segment, issued by the thread that
+// holds the candidate's id: a bulk copy costs its SM some 33 cycles whatever its size, so only the widest CTAs, where
+// the arithmetic per candidate exceeds that, gain by the instructions it saves; the probabilities of a tile pass through registers into shared memory, each written
+// twice side by side ([j][head] pairs, pitch +16 bytes: the stores of 8 candidates x 2 heads fall into different
+// banks), so that one 16-byte load gives the factor pairs of two heads.  Per candidate a thread issues HG / 2 + 1
+// shared loads for HG * NPAIR packed multiply-adds.
 #define PVS_NS 3
-// HG heads x NP channel pairs per CTA (NP threads), T candidates per staged tile
-template <bool BF16, int HG, int NP, int T>
-__global__ void __launch_bounds__(NP)
+__device__ int g_attn_status = 0;         // 31: a row copy did not arrive within the wait's budget
+template <bool BF16, int HG, int NPAIR, int T, int NT, bool BULK>
+struct PvCfg {
+    static constexpr int ROWB = NT * NPAIR * (BF16 ? 4 : 8);     // bytes of a row's segment
+    static constexpr int PP = HG * 8 + 16;                       // bytes per candidate of the probability tile
+    static constexpr int STAGE = T * (ROWB + PP), SMEM = PVS_NS * STAGE + (BULK ? 0 : 4 * T * 4);
+};
+
+// The operands of GJ candidates for a thread: its channel pairs and the factor pairs of the heads
+template <bool BF16, int HG, int NPAIR, int GJ, int ROWB, int PP>
+struct PvOps {
+    uint32_t w[GJ][BF16 ? NPAIR : 1];
+    ulonglong2 v[GJ][BF16 ? 1 : (NPAIR + 1) / 2], p[GJ][HG / 2];
+    __device__ __forceinline__ void load(const unsigned char *rows, const unsigned char *sp, int j0, int tid) {
+#pragma unroll
+        for (int u = 0; u < GJ; u++) {
+            const unsigned char *r = rows + (size_t)(j0 + u) * ROWB + tid * (NPAIR * (BF16 ? 4 : 8));
+            if constexpr (BF16 && NPAIR == 2) {
+                const uint2 x = *reinterpret_cast<const uint2 *>(r);
+                w[u][0] = x.x; w[u][1] = x.y;
+            } else if constexpr (BF16) {
+                w[u][0] = *reinterpret_cast<const uint32_t *>(r);
+            } else if constexpr (NPAIR == 2) {
+                v[u][0] = *reinterpret_cast<const ulonglong2 *>(r);
+            } else {
+                v[u][0].x = *reinterpret_cast<const f32x2 *>(r);
+            }
+#pragma unroll
+            for (int a = 0; a < HG / 2; a++) p[u][a] = *reinterpret_cast<const ulonglong2 *>(sp + (size_t)(j0 + u) * PP + a * 16);
+        }
+    }
+    template <bool FUSED>
+    __device__ __forceinline__ void walk(f32x2 (&acc)[HG][NPAIR]) const {
+#pragma unroll
+        for (int u = 0; u < GJ; u++)
+#pragma unroll
+            for (int i = 0; i < NPAIR; i++) {
+                f32x2 x;
+                if constexpr (BF16) x = pack2(__uint_as_float(w[u][i] << 16), __uint_as_float(w[u][i] & 0xffff0000u));
+                else x = i ? v[u][0].y : v[u][0].x;
+#pragma unroll
+                for (int a = 0; a < HG; a++) acc[a][i] = mac2<FUSED>(acc[a][i], a & 1 ? p[u][a >> 1].y : p[u][a >> 1].x, x);
+            }
+    }
+};
+// A tile of T candidates (cnt of them in the row); the operands are read GJ candidates ahead of their use
+template <bool BF16, bool FUSED, int HG, int NPAIR, int T, int ROWB, int PP>
+__device__ __forceinline__ void pv_tile(f32x2 (&acc)[HG][NPAIR], const unsigned char *rows, const unsigned char *sp, int cnt, int tid) {
+    constexpr int GJ = HG * NPAIR >= 16 ? 1 : HG * NPAIR >= 8 ? 2 : 4;
+    if (cnt == T) {
+        PvOps<BF16, HG, NPAIR, GJ, ROWB, PP> A, B;
+        A.load(rows, sp, 0, tid);
+#pragma unroll 2
+        for (int j = 0; j < T; j += 2 * GJ) {
+            B.load(rows, sp, j + GJ, tid);
+            A.template walk<FUSED>(acc);
+            if (j + 2 * GJ < T) A.load(rows, sp, j + 2 * GJ, tid);
+            B.template walk<FUSED>(acc);
+        }
+    } else {
+        PvOps<BF16, HG, NPAIR, 1, ROWB, PP> A;
+        for (int j = 0; j < cnt; j++) { A.load(rows, sp, j, tid); A.template walk<FUSED>(acc); }
+    }
+}
+
+template <bool BF16, int HG, int NPAIR, int T, int NT, bool BULK>
+__global__ void __launch_bounds__(NT)
 sparse_pv_stage_kernel(const float *__restrict__ p, const float *__restrict__ den, int h, int d,
                        const int32_t *__restrict__ ids, const int *__restrict__ ns, int idxw, const void *kv_a, int64_t na,
-                       const void *kv_b, float *__restrict__ o, size_t a_stride, size_t b_stride, int seq_mod, const SaRope rope) {
+                       const void *kv_b, float *__restrict__ o, size_t a_stride, size_t b_stride, int seq_mod, const SaRope rope,
+                       const int *__restrict__ bad) {
     APUS_PDL_WAIT();
     APUS_PDL_GO();
-    constexpr int ROWB = NP * (BF16 ? 4 : 8);              // bytes of a row's segment
-    constexpr int CPR = ROWB / 16;                             // 16-byte copies per row
-    constexpr int STAGE = T * ROWB + T * HG * 4;       // rows, then the tile's probabilities [T][HG]
+    using Cf = PvCfg<BF16, HG, NPAIR, T, NT, BULK>;
+    constexpr int ROWB = Cf::ROWB, PP = Cf::PP, STAGE = Cf::STAGE, CPR = ROWB / 16;
+    constexpr int NP = T * HG / NT;                         // probabilities of a tile per thread
+    static_assert(T * HG % NT == 0 && T <= NT && HG % 2 == 0 && ROWB % 16 == 0 && STAGE % 16 == 0, "tile shape");
     extern __shared__ __align__(16) unsigned char pvs[];
+    __shared__ uint64_t s_full[PVS_NS];
+    __shared__ volatile int s_abort;
     const int t = blockIdx.y, h0 = (int)blockIdx.x * HG, tid = threadIdx.x;
-    const int k2 = (int)blockIdx.z * NP + tid;             // this thread's channel pair
     const int own = seq_mod > 0 ? t % seq_mod : t;
-    const size_t esz = BF16 ? 2 : 4;
+    const size_t rowsz = (size_t)d * (BF16 ? 2 : 4);
     const char *base_a = reinterpret_cast<const char *>(kv_a) + (size_t)own * a_stride + (size_t)blockIdx.z * ROWB;
-    const char *base_b = reinterpret_cast<const char *>(kv_b) + (size_t)own * b_stride + (size_t)blockIdx.z * ROWB;
+    const char *base_b = reinterpret_cast<const char *>(kv_b) + (size_t)own * b_stride + (size_t)blockIdx.z * ROWB - (size_t)na * rowsz;
     const int n = ns[t];
+    const bool fused = bad[t] == 0;
     const int32_t *idr = ids + (size_t)t * idxw;
     const int ntile = (n + T - 1) / T;
-    auto stage = [&](int c) {
-        if (c < ntile) {
-            unsigned char *st = pvs + (size_t)(c % PVS_NS) * STAGE;
-            const int j0 = c * T, cnt = min(T, n - j0);
-#pragma unroll 4
-            for (int i = tid; i < T * CPR; i += NP) {
-                const int r = i / CPR, seg = i - r * CPR;
-                if (r < cnt) {
-                    const int32_t id = idr[j0 + r];
-                    const char *src = id < na ? base_a + (size_t)id * d * esz : base_b + (size_t)(id - na) * d * esz;
-                    cp_async16(st + (size_t)r * ROWB + seg * 16, src + seg * 16, true);
+    auto id_load = [&](int c) { const int j = c * T + tid; return tid < T && j < n ? idr[j] : -1; };
+    // tile c's segments.  BULK: thread r copies the one of candidate c T + r (id < 0: past the row's end); otherwise the
+    // ids pass through shared memory and every thread copies its 16-byte column of every NT / CPR-th row
+    int32_t *s_id = reinterpret_cast<int32_t *>(pvs + (size_t)PVS_NS * STAGE);       // [4][T]
+    auto id_store = [&](int c, int32_t v) { if (!BULK && tid < T) s_id[(c & 3) * T + tid] = v; };
+    auto stage = [&](int c, int32_t id) {
+        if constexpr (!BULK) {
+            static_assert(BULK || (NT % CPR == 0 && T * CPR % NT == 0), "copies must divide among the threads");
+            if (c < ntile) {
+                unsigned char *st = pvs + (size_t)(c % PVS_NS) * STAGE;
+                const int cnt = min(T, n - c * T), seg = tid % CPR;
+#pragma unroll 8
+                for (int i = 0; i < T * CPR / NT; i++) {
+                    const int r = tid / CPR + i * (NT / CPR);
+                    if (r < cnt) {
+                        const int32_t rid = s_id[(c & 3) * T + r];
+                        cp_async16(st + (size_t)r * ROWB + seg * 16, (rid < na ? base_a : base_b) + (size_t)rid * rowsz + seg * 16, true);
+                    }
                 }
             }
-            for (int i = tid; i < T * HG; i += NP) {
-                const int r = i / HG, a = i - r * HG;
-                if (r < cnt && h0 + a < h) {
-                    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(st + T * ROWB + i * 4);
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(p + ((size_t)t * h + h0 + a) * idxw + j0 + r) : "memory");
-                } else {
-                    *reinterpret_cast<float *>(st + T * ROWB + i * 4) = 0.f;
-                }
-            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            return;
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (c >= ntile || tid >= T) return;
+        uint64_t *bar = &s_full[c % PVS_NS];
+        if (id >= 0) {
+            mbar_expect_tx(bar, ROWB);
+            bulk_load(pvs + (size_t)(c % PVS_NS) * STAGE + (size_t)tid * ROWB, (id < na ? base_a : base_b) + (size_t)id * rowsz, ROWB, bar);
+        } else {
+            mbar_arrive(bar);
+        }
     };
-    float a0[HG], a1[HG];
+    // probability u of this thread: head 2 (i / 2T) + i % 2, candidate (i / 2) % T with i = tid + NT u
+    float preg[NP];
+    auto p_load = [&](int c) {
 #pragma unroll
-    for (int a = 0; a < HG; a++) a0[a] = a1[a] = 0.f;
-    stage(0);
-    stage(1);
+        for (int u = 0; u < NP; u++) {
+            const int i = tid + NT * u, a = 2 * (i / (2 * T)) + (i & 1), j = c * T + (i >> 1) % T;
+            preg[u] = j < n && h0 + a < h ? p[((size_t)t * h + h0 + a) * idxw + j] : 0.f;
+        }
+    };
+    auto p_store = [&](int c) {
+        unsigned char *sp = pvs + (size_t)(c % PVS_NS) * STAGE + T * ROWB;
+#pragma unroll
+        for (int u = 0; u < NP; u++) {
+            const int i = tid + NT * u, a = 2 * (i / (2 * T)) + (i & 1), j = (i >> 1) % T;
+            *reinterpret_cast<f32x2 *>(sp + (size_t)j * PP + a * 8) = pack2(preg[u], preg[u]);
+        }
+    };
+    f32x2 acc[HG][NPAIR];
+#pragma unroll
+    for (int a = 0; a < HG; a++)
+#pragma unroll
+        for (int i = 0; i < NPAIR; i++) acc[a][i] = 0ull;
+    if (tid == 0) {
+        for (int i = 0; i < PVS_NS; i++) mbar_init(&s_full[i], T);
+        s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    int32_t id_next = id_load(2);                              // one tile ahead of the copies that need it
+    p_load(0);
+    const int32_t id0 = id_load(0), id1 = id_load(1);
+    id_store(0, id0);
+    id_store(1, id1);
+    id_store(2, id_next);
+    __syncthreads();
+    stage(0, id0);
+    stage(1, id1);
+    p_store(0);
+    int fail = 0;
     for (int c = 0; c < ntile; c++) {
-        stage(c + 2);                                          // its buffer was consumed at step c - 1, behind that step's barrier
-        asm volatile("cp.async.wait_group 2;" ::: "memory");
-        __syncthreads();                                       // tile c of every thread has landed
+        const int32_t id_after = id_load(c + 3);
+        if constexpr (BULK) {
+            fail = !mbar_wait(&s_full[c % PVS_NS], (uint32_t)(c / PVS_NS) & 1u, &s_abort);
+            if (__syncthreads_or(fail)) { fail = 1; break; }   // tile c has landed for every thread, tile c - 1 is consumed
+        } else {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();
+        }
+        stage(c + 2, id_next);
+        id_next = id_after;
+        if (c + 1 < ntile) p_load(c + 1);
         const unsigned char *st = pvs + (size_t)(c % PVS_NS) * STAGE;
-        const float4 *sp = reinterpret_cast<const float4 *>(st + T * ROWB);
         const int cnt = min(T, n - c * T);
-#pragma unroll 4
-        for (int j = 0; j < cnt; j++) {
-            float2 v;
-            if (BF16) {
-                const uint32_t w = *reinterpret_cast<const uint32_t *>(st + (size_t)j * ROWB + tid * 4);
-                v = make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
-            } else {
-                v = *reinterpret_cast<const float2 *>(st + (size_t)j * ROWB + tid * 8);
-            }
-#pragma unroll
-            for (int m = 0; m < HG / 4; m++) {
-                const float4 p4 = sp[j * (HG / 4) + m];
-                const float pa[4] = {p4.x, p4.y, p4.z, p4.w};
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    a0[4 * m + e] = __fadd_rn(a0[4 * m + e], __fmul_rn(pa[e], v.x));
-                    a1[4 * m + e] = __fadd_rn(a1[4 * m + e], __fmul_rn(pa[e], v.y));
-                }
-            }
-        }
-        __syncthreads();                                       // this tile's buffer is free again
+        if (fused) pv_tile<BF16, true, HG, NPAIR, T, ROWB, PP>(acc, st, st + T * ROWB, cnt, tid);
+        else pv_tile<BF16, false, HG, NPAIR, T, ROWB, PP>(acc, st, st + T * ROWB, cnt, tid);
+        if (c + 1 < ntile) p_store(c + 1);                     // this stage was consumed at tile c - 2
+        id_store(c + 3, id_after);                             // slot of tile c - 1, whose copies are all issued
     }
-    const int ri = rope.cs ? k2 - (d - rope.rd) / 2 : -1;
-    float co = 1.f, si = 0.f;
-    if (ri >= 0) {
-        const float *c = rope.cs + (rope.pos ? (size_t)*rope.pos * rope.rd : 0);
-        co = c[ri]; si = -c[rope.rd / 2 + ri];
+    if (fail) {
+        if (tid == 0) atomicCAS(&g_attn_status, 0, 31);
+        for (int i = 0; i < 2000; i++) __nanosleep(1000);      // copies already issued to this CTA's shared memory land
+        return;
     }
 #pragma unroll
-    for (int a = 0; a < HG; a++) {
-        if (h0 + a >= h) continue;
-        float *ov = o + ((size_t)t * h + h0 + a) * d;
-        if (n == 0) { ov[2 * k2] = 0.f; ov[2 * k2 + 1] = 0.f; continue; }
-        const float dn = den[(size_t)t * h + h0 + a];
-        float x1 = bf16_round(__fdiv_rn(a0[a], dn)), x2 = bf16_round(__fdiv_rn(a1[a], dn));
+    for (int i = 0; i < NPAIR; i++) {
+        const int k2 = ((int)blockIdx.z * NT + tid) * NPAIR + i;       // this channel pair
+        const int ri = rope.cs ? k2 - (d - rope.rd) / 2 : -1;
+        float co = 1.f, si = 0.f;
         if (ri >= 0) {
-            const float y1 = bf16_round(__fsub_rn(__fmul_rn(x1, co), __fmul_rn(x2, si)));
-            const float y2 = bf16_round(__fadd_rn(__fmul_rn(x1, si), __fmul_rn(x2, co)));
-            x1 = y1; x2 = y2;
+            const float *c = rope.cs + (rope.pos ? (size_t)*rope.pos * rope.rd : 0);
+            co = c[ri]; si = -c[rope.rd / 2 + ri];
         }
-        ov[2 * k2] = x1;
-        ov[2 * k2 + 1] = x2;
+#pragma unroll
+        for (int a = 0; a < HG; a++) {
+            if (h0 + a >= h) continue;
+            float *ov = o + ((size_t)t * h + h0 + a) * d + 2 * k2;
+            if (n == 0) { ov[0] = 0.f; ov[1] = 0.f; continue; }
+            const float dn = den[(size_t)t * h + h0 + a];
+            const float2 s = unpack2(acc[a][i]);
+            float x1 = bf16_round(__fdiv_rn(s.x, dn)), x2 = bf16_round(__fdiv_rn(s.y, dn));
+            if (ri >= 0) {
+                const float y1 = bf16_round(__fsub_rn(__fmul_rn(x1, co), __fmul_rn(x2, si)));
+                const float y2 = bf16_round(__fadd_rn(__fmul_rn(x1, si), __fmul_rn(x2, co)));
+                x1 = y1; x2 = y2;
+            }
+            if (((uintptr_t)o & 7) == 0) *reinterpret_cast<float2 *>(ov) = make_float2(x1, x2);
+            else { ov[0] = x1; ov[1] = x2; }
+        }
     }
 }
 
 // Drops negative ids keeping order (reference c/attn.h:1314-1321).
 __global__ void compact_ids_kernel(const int32_t *__restrict__ idxs, int idxw,
-                                   int32_t *__restrict__ out, int *__restrict__ ns) {
+                                   int32_t *__restrict__ out, int *__restrict__ ns, int *__restrict__ bad) {
     APUS_PDL_WAIT();
     APUS_PDL_GO();
     __shared__ int s_base;
@@ -842,7 +1042,7 @@ __global__ void compact_ids_kernel(const int32_t *__restrict__ idxs, int idxw,
         if (tid == 0) s_base += total;
         __syncthreads();
     }
-    if (tid == 0) ns[t] = s_base;
+    if (tid == 0) { ns[t] = s_base; bad[t] = 0; }
 }
 
 // Scores / compacted ids between the kernels of a call: the caller's scratch (a model
@@ -861,10 +1061,104 @@ static void *ensure_scratch(size_t bytes) {
     g_scratch_cap = bytes;
     return g_scratch;
 }
-size_t sparse_attn_scratch(int h, int idxw, int s) {
-    const size_t sc_bytes = (size_t)s * h * idxw * sizeof(float), ids_bytes = (size_t)s * idxw * sizeof(int32_t);
-    const size_t ns_off = (sc_bytes + ids_bytes + 255) & ~(size_t)255;
-    return ((ns_off + (size_t)s * sizeof(int) + 255) & ~(size_t)255) + (size_t)s * h * sizeof(float);
+// Layout of that scratch: scores, compacted ids, their counts, denominators, the walk flags of P.V.
+struct SaScratch {
+    size_t ids, ns, den, bad, bytes;
+    SaScratch(int h, int idxw, int s) {
+        ids = (size_t)s * h * idxw * sizeof(float);
+        ns = (ids + (size_t)s * idxw * sizeof(int32_t) + 255) & ~(size_t)255;
+        den = (ns + (size_t)s * sizeof(int) + 255) & ~(size_t)255;
+        bad = den + (size_t)s * h * sizeof(float);
+        bytes = bad + (size_t)s * sizeof(int);
+    }
+};
+size_t sparse_attn_scratch(int h, int idxw, int s) { return SaScratch(h, idxw, s).bytes; }
+
+int attn_status(int reset) {
+    int v = 0;
+    if (cudaMemcpyFromSymbol(&v, g_attn_status, sizeof(int)) != cudaSuccess) return -1;
+    if (reset && v) {
+        int z = 0;
+        cudaMemcpyToSymbol(g_attn_status, &z, sizeof(int));
+    }
+    return v;
+}
+
+// ---- launches of the tiled kernels ----
+template <bool BF16, int HL, int CL, int WH, int WC>
+static int scores_launch(const float *q, int h, int d, const int32_t *ids, const int *ns, int idxw, int s, float scale,
+                         const void *kv_a, int64_t na, const void *kv_b, float *sc, int *bad, cudaStream_t st, size_t sa,
+                         size_t sb, int seq_mod) {
+    using Cf = ScoreCfg<BF16, HL, CL, WH, WC>;
+    auto kern = sparse_scores_tile_kernel<BF16, HL, CL, WH, WC>;
+    if (ensure_dyn_smem((const void *)kern, Cf::SMEM + 64)) return 1;
+    launch_k(kern, dim3((unsigned)ceil_div(idxw, Cf::CANDS), (unsigned)ceil_div(h, Cf::HEADS), (unsigned)s), Cf::THREADS, Cf::SMEM,
+             st, q, h, d, ids, ns, idxw, scale, kv_a, na, kv_b, sc, sa, sb, seq_mod, bad);
+    APUS_LAUNCHED();
+    return 0;
+}
+template <bool BF16, int HG, int NPAIR, int T, int NT, bool BULK>
+static int pv_launch(const float *sc, const float *den, int h, int d, const int32_t *ids, const int *ns, int idxw, int s,
+                     const void *kv_a, int64_t na, const void *kv_b, float *o, const int *bad, cudaStream_t st, size_t sa,
+                     size_t sb, int seq_mod, const SaRope &rope) {
+    using Cf = PvCfg<BF16, HG, NPAIR, T, NT, BULK>;
+    auto kern = sparse_pv_stage_kernel<BF16, HG, NPAIR, T, NT, BULK>;
+    if (ensure_dyn_smem((const void *)kern, Cf::SMEM + 64)) return 1;
+    launch_k(kern, dim3((unsigned)ceil_div(h, HG), (unsigned)s, (unsigned)(d / (2 * NPAIR * NT))), NT, Cf::SMEM, st,
+             sc, den, h, d, ids, ns, idxw, kv_a, na, kv_b, o, sa, sb, seq_mod, rope, bad);
+    APUS_LAUNCHED();
+    return 0;
+}
+template <bool BF16>
+static int attn_tiled(const float *q, const float *sink, int h, int d, const int32_t *ids, const int *ns, int idxw, int s,
+                      float scale, const void *kv_a, int64_t na, const void *kv_b, float *sc, float *den, int *bad, float *o,
+                      cudaStream_t st, size_t sa, size_t sb, int seq_mod, const SaRope &rope) {
+#define SA_ARGS q, h, d, ids, ns, idxw, s, scale, kv_a, na, kv_b, sc, bad, st, sa, sb, seq_mod
+    // The larger a lane's tile, the fewer shared loads per multiply-add; the smaller, the more warps share the work
+    // of a small step.  Lines drawn where the measured times cross (64 heads, d = 512, BF16 rows; us with 16 heads x
+    // 32 candidates of 4 x 1 per lane / 16 x 32 of 4 x 2 / 64 x 64 of 4 x 4): 1 row of 640 candidates 11.6 / 15.0 /
+    // 25.1, 2 rows 16.4 / 15.6 / 25.4, 4 rows 20.8 / 19.2 / 25.6, 7 rows of 909 38 / 26.7 / 26.0, 32 rows of 640
+    // 107 / 76 / 62 (96 before).
+    const long long c64 = (long long)ceil_div(idxw, 64) * ceil_div(h, 64) * s;
+    if (c64 < 15) { if (scores_launch<BF16, 4, 1, 1, 4>(SA_ARGS)) return 1; }
+    else if (c64 < 80) { if (scores_launch<BF16, 4, 2, 1, 2>(SA_ARGS)) return 1; }
+    else if (scores_launch<BF16, 4, 4, 4, 2>(SA_ARGS)) return 1;
+#undef SA_ARGS
+    // a warp per row once that is a warp and more for every scheduler; with fewer rows the exponentials want a CTA per
+    // row (64 rows of 640: 5.1 us against 7.9, 448 of 909: 7.8 / 11, 2,048 of 640: 12.2 / 10.6)
+    if (idxw <= 1024 && (long long)s * h >= 1024) {
+        const size_t sm = (size_t)8 * ((idxw + 3) & ~3) * sizeof(float);
+        launch_k(sparse_softmax_rows_kernel, dim3((unsigned)ceil_div(h, 8), (unsigned)s), 256, sm, st, sc, sink, h, ns, idxw, den, bad);
+    } else {
+        const size_t sm2 = (size_t)idxw * sizeof(float);
+        if (ensure_dyn_smem((const void *)sparse_softmax_kernel, sm2 + 256)) return 1;
+        launch_k(sparse_softmax_kernel, dim3((unsigned)h, (unsigned)s), 256, sm2, st, sc, sink, h, ns, idxw, den, bad);
+    }
+    APUS_LAUNCHED();
+    if (d % 256 == 0) {
+        // Few rows: few heads per CTA and short chains of instructions per candidate; many rows: many heads per
+        // gathered row.  Lines drawn where the measured times cross (64 heads, d = 512, BF16 rows of 640; us with 2 / 4 /
+        // 4 / 8 / 8 heads per CTA as listed): 1 row 15.8 / 18.0 / 22.0 / 29.1 / 52.0 (42.6 before), 4 rows 20.4 / 19.3 /
+        // 23.3 / 29.5 / 52.1, 12 rows 57 / 44 / 36 / 41 / 53, 16 rows 74 / 59 / 44 / 41 / 53, 32 rows 131 / 99 / 81 / 76 /
+        // 63 (94 before).  The last takes rows of 512 channels, with 256 its CTA is half as wide.
+        const long long w16 = (long long)s * ceil_div(h, 16) * (d / 128);
+#define PV_ARGS sc, den, h, d, ids, ns, idxw, s, kv_a, na, kv_b, o, bad, st, sa, sb, seq_mod, rope
+        if (w16 <= 32) return pv_launch<BF16, 2, 1, 64, 64, false>(PV_ARGS);
+        if (w16 <= 64) return pv_launch<BF16, 4, 1, 64, 64, false>(PV_ARGS);
+        if (w16 <= 224) return pv_launch<BF16, 4, 1, 32, 64, false>(PV_ARGS);
+        if (w16 <= 352) return pv_launch<BF16, 8, 1, 32, 128, false>(PV_ARGS);
+        if (d % 512 == 0) return pv_launch<BF16, 8, 2, 16, 128, true>(PV_ARGS);
+        return pv_launch<BF16, 8, 2, (BF16 ? 32 : 16), 64, true>(PV_ARGS);
+#undef PV_ARGS
+    }
+    if (h >= 16 && (long long)s * ceil_div(h, 16) >= 96)
+        launch_k(sparse_pv_tile_kernel<BF16, 16>, dim3((unsigned)ceil_div(h, 16), (unsigned)s), 256, 0, st, sc, den, h, d, ids, ns,
+                 idxw, kv_a, na, kv_b, o, sa, sb, seq_mod, rope);
+    else
+        launch_k(sparse_pv_tile_kernel<BF16, 4>, dim3((unsigned)ceil_div(h, 4), (unsigned)s), 256, 0, st, sc, den, h, d, ids, ns,
+                 idxw, kv_a, na, kv_b, o, sa, sb, seq_mod, rope);
+    APUS_LAUNCHED();
+    return 0;
 }
 
 int sparse_attn(const float *q, const float *sink, int h, int d,
@@ -878,88 +1172,26 @@ int sparse_attn(const float *q, const float *sink, int h, int d,
     APUS_REQUIRE(d % 2 == 0 && d <= 1024, "sparse_attn: d=%d unsupported", d);
     APUS_REQUIRE((size_t)idxw * sizeof(float) <= 160 * 1024, "sparse_attn: idxw=%d too wide", idxw);
     if (s <= 0 || idxw <= 0) return 0;
-    size_t sc_bytes = (size_t)s * h * idxw * sizeof(float);
-    size_t ids_bytes = (size_t)s * idxw * sizeof(int32_t);
-    size_t ns_off = (sc_bytes + ids_bytes + 255) & ~(size_t)255;
-    const size_t den_off = (ns_off + (size_t)s * sizeof(int) + 255) & ~(size_t)255;
-    const size_t need = den_off + (size_t)s * h * sizeof(float);
-    APUS_REQUIRE(!callers || need <= callers_cap, "sparse_attn: scratch of %zu bytes given, %zu needed", callers_cap, need);
-    void *scratch = callers ? callers : ensure_scratch(need);
+    const SaScratch lay(h, idxw, s);
+    APUS_REQUIRE(!callers || lay.bytes <= callers_cap, "sparse_attn: scratch of %zu bytes given, %zu needed", callers_cap, lay.bytes);
+    char *scratch = (char *)(callers ? callers : ensure_scratch(lay.bytes));
     if (!scratch) return 1;
     float *sc = (float *)scratch;
-    int32_t *ids = (int32_t *)((char *)scratch + sc_bytes);
-    int *ns = (int *)((char *)scratch + ns_off);
-    float *den = (float *)((char *)scratch + den_off);
+    int32_t *ids = (int32_t *)(scratch + lay.ids);
+    int *ns = (int *)(scratch + lay.ns);
+    float *den = (float *)(scratch + lay.den);
+    int *bad = (int *)(scratch + lay.bad);
     APUS_REQUIRE(!ids_ready || callers, "sparse_attn: compacted ids need the caller's scratch");
     if (!ids_ready) {
-        launch_k(compact_ids_kernel, s, 256, 0, st, idxs, idxw, ids, ns);
+        launch_k(compact_ids_kernel, s, 256, 0, st, idxs, idxw, ids, ns, bad);
         APUS_LAUNCHED();
     }
     const SaRope no_rope = {nullptr, nullptr, 0};
     static const int tiled = [] { const char *e = getenv("APUS_ATTN_TILED"); return !(e && e[0] == '0'); }();
     if (tiled && d % 64 == 0) {
-        // register-tiled kernels: enough CTAs to cover the SMs decide the tile sizes
-        const long long wide = (long long)ceil_div(idxw, 256) * ceil_div(h, 16) * s;
-        const size_t sm2 = (size_t)idxw * sizeof(float);
-        if (ensure_dyn_smem((const void *)sparse_softmax_kernel, sm2)) return 1;
-        const int hgs = h >= 16 && (long long)s * ceil_div(h, 16) >= 96 ? 16 : 4;
-        const size_t kc = kv_bf16 ? 64 : 32;
-        const size_t ss8 = 2 * kc * 16 * 4 + 8 * (2 * 32 * SS_PITCHW * 4), ss2 = 2 * kc * 16 * 4 + 2 * (2 * 32 * SS_PITCHW * 4);
-        const size_t ss1 = 2 * kc * 16 * 4 + 2 * (2 * 8 * SS_PITCHW * 4);
-        // a small step (few rows, few candidates): 8-candidate tiles, so that no warp walks more than a quarter
-        static const bool small_on = [] { const char *e = getenv("APUS_ATTN_SMALL"); return !(e && e[0] == '0'); }();
-        const bool narrow = small_on && (long long)ceil_div(idxw, 32) * ceil_div(h, 16) * s <= 296;
-        // P.V from staged rows where the row splits into whole CTAs' worth of channel pairs: 16 heads x 128 pairs
-        // per CTA when there are (row, 16 heads) groups enough to fill the GPU, else 4 heads x 64 pairs
-        static const bool stage_on = [] { const char *e = getenv("APUS_ATTN_STAGE"); return !(e && e[0] == '0'); }();
-        const bool pv_stage = stage_on && d % 256 == 0;
-        const size_t rowb = kv_bf16 ? 4 : 8;
-        const size_t pvs4 = (size_t)PVS_NS * (64 * 64 * rowb + 64 * 4 * 4);
-        const size_t pvs16 = (size_t)PVS_NS * ((kv_bf16 ? 64 : 32) * 128 * rowb + (kv_bf16 ? 64 : 32) * 16 * 4);
-        if (pv_stage && (ensure_dyn_smem(kv_bf16 ? (const void *)sparse_pv_stage_kernel<true, 4, 64, 64>
-                                                 : (const void *)sparse_pv_stage_kernel<false, 4, 64, 64>, pvs4) ||
-                         ensure_dyn_smem(kv_bf16 ? (const void *)sparse_pv_stage_kernel<true, 16, 128, 64>
-                                                 : (const void *)sparse_pv_stage_kernel<false, 16, 128, 32>, pvs16)))
-            return 1;
-        if (ensure_dyn_smem(kv_bf16 ? (const void *)sparse_scores_tile_kernel<true, 8, 4> : (const void *)sparse_scores_tile_kernel<false, 8, 4>, ss8))
-            return 1;
-#define APUS_SA_LAUNCH(BF)                                                                                              \
-        do {                                                                                                            \
-            if (wide >= 148) {                                                                                          \
-                dim3 g((unsigned)ceil_div(idxw, 256), (unsigned)ceil_div(h, 16), (unsigned)s);                          \
-                launch_k(sparse_scores_tile_kernel<BF, 8, 4>, g, 256, ss8, st, q, h, d, ids, ns, idxw, scale, kv_a, na, kv_b, sc,  \
-                                                                   sa, sb, seq_mod);                                    \
-            } else if (narrow) {                                                                                        \
-                dim3 g((unsigned)ceil_div(idxw, 16), (unsigned)ceil_div(h, 16), (unsigned)s);                           \
-                launch_k(sparse_scores_tile_kernel<BF, 2, 1>, g, 64, ss1, st, q, h, d, ids, ns, idxw, scale, kv_a, na, kv_b, sc,   \
-                                                                  sa, sb, seq_mod);                                     \
-            } else {                                                                                                    \
-                dim3 g((unsigned)ceil_div(idxw, 64), (unsigned)ceil_div(h, 16), (unsigned)s);                           \
-                launch_k(sparse_scores_tile_kernel<BF, 2, 4>, g, 64, ss2, st, q, h, d, ids, ns, idxw, scale, kv_a, na, kv_b, sc,   \
-                                                                  sa, sb, seq_mod);                                     \
-            }                                                                                                           \
-            APUS_LAUNCHED();                                                                                            \
-            launch_k(sparse_softmax_kernel, dim3((unsigned)h, (unsigned)s), 256, sm2, st, sc, sink, h, ns, idxw, den);       \
-            APUS_LAUNCHED();                                                                                            \
-            if (pv_stage && hgs == 16)                                                                                  \
-                launch_k(sparse_pv_stage_kernel<BF, 16, 128, (BF ? 64 : 32)>,                                           \
-                    dim3((unsigned)ceil_div(h, 16), (unsigned)s, (unsigned)(d / 2 / 128)), 128, pvs16, st,              \
-                    sc, den, h, d, ids, ns, idxw, kv_a, na, kv_b, o, sa, sb, seq_mod, rope ? *rope : no_rope);          \
-            else if (pv_stage)                                                                                          \
-                launch_k(sparse_pv_stage_kernel<BF, 4, 64, 64>,                                                         \
-                    dim3((unsigned)ceil_div(h, 4), (unsigned)s, (unsigned)(d / 2 / 64)), 64, pvs4, st,                  \
-                    sc, den, h, d, ids, ns, idxw, kv_a, na, kv_b, o, sa, sb, seq_mod, rope ? *rope : no_rope);          \
-            else if (hgs == 16)                                                                                         \
-                launch_k(sparse_pv_tile_kernel<BF, 16>, dim3((unsigned)ceil_div(h, 16), (unsigned)s), 256, 0, st,             \
-                    sc, den, h, d, ids, ns, idxw, kv_a, na, kv_b, o, sa, sb, seq_mod, rope ? *rope : no_rope);          \
-            else                                                                                                        \
-                launch_k(sparse_pv_tile_kernel<BF, 4>, dim3((unsigned)ceil_div(h, 4), (unsigned)s), 256, 0, st,               \
-                    sc, den, h, d, ids, ns, idxw, kv_a, na, kv_b, o, sa, sb, seq_mod, rope ? *rope : no_rope);          \
-            APUS_LAUNCHED();                                                                                            \
-        } while (0)
-        if (kv_bf16) APUS_SA_LAUNCH(true); else APUS_SA_LAUNCH(false);
-#undef APUS_SA_LAUNCH
-        return 0;
+        const SaRope rp = rope ? *rope : no_rope;
+        return kv_bf16 ? attn_tiled<true>(q, sink, h, d, ids, ns, idxw, s, scale, kv_a, na, kv_b, sc, den, bad, o, st, sa, sb, seq_mod, rp)
+                       : attn_tiled<false>(q, sink, h, d, ids, ns, idxw, s, scale, kv_a, na, kv_b, sc, den, bad, o, st, sa, sb, seq_mod, rp);
     }
     size_t sm1 = ((size_t)SA_IDS * (d + 1) + (size_t)SA_HEADS * d) * sizeof(float);
     dim3 g1((unsigned)ceil_div(idxw, SA_IDS), (unsigned)ceil_div(h, SA_HEADS), (unsigned)s);
@@ -991,11 +1223,11 @@ int sparse_attn(const float *q, const float *sink, int h, int d,
 
 int sparse_attn_compact(const int32_t *idxs, int h, int idxw, int s, void *scratch, size_t scratch_cap, cudaStream_t st) {
     if (s <= 0 || idxw <= 0) return 0;
-    APUS_REQUIRE(scratch && sparse_attn_scratch(h, idxw, s) <= scratch_cap, "sparse_attn_compact: scratch of %zu bytes given, %zu needed",
-                 scratch_cap, sparse_attn_scratch(h, idxw, s));
-    const size_t sc_bytes = (size_t)s * h * idxw * sizeof(float), ids_bytes = (size_t)s * idxw * sizeof(int32_t);
-    const size_t ns_off = (sc_bytes + ids_bytes + 255) & ~(size_t)255;
-    launch_k(compact_ids_kernel, s, 256, 0, st, idxs, idxw, (int32_t *)((char *)scratch + sc_bytes), (int *)((char *)scratch + ns_off));
+    const SaScratch lay(h, idxw, s);
+    APUS_REQUIRE(scratch && lay.bytes <= scratch_cap, "sparse_attn_compact: scratch of %zu bytes given, %zu needed", scratch_cap,
+                 lay.bytes);
+    char *p = (char *)scratch;
+    launch_k(compact_ids_kernel, s, 256, 0, st, idxs, idxw, (int32_t *)(p + lay.ids), (int *)(p + lay.ns), (int *)(p + lay.bad));
     APUS_LAUNCHED();
     return 0;
 }

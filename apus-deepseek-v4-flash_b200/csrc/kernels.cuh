@@ -201,6 +201,7 @@ int sparse_attn(const float *q, const float *sink, int h, int d,
                 bool ids_ready = false,              // sparse_attn_compact has run on this scratch with these index rows
                 const struct SaRope *rope = nullptr);   // rotate the output rows back before they are written
 size_t sparse_attn_scratch(int h, int idxw, int s);
+int attn_status(int reset);               // status word of the bounded waits in P.V (0 = none expired)
 // The first launch of sparse_attn (negative ids dropped, order kept) on its own: a caller that has the
 // index rows before the queries (a side chain) runs it there, into the scratch it then hands to sparse_attn.
 int sparse_attn_compact(const int32_t *idxs, int h, int idxw, int s, void *scratch, size_t scratch_cap, cudaStream_t st);

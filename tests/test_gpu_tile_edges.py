@@ -1,13 +1,59 @@
 """The tiled kernels at the edges of their tiles and on both sides of their dispatch rules, bit for bit against a
-kernel of this library that knows no tiles."""
+kernel of this library that knows no tiles: sparse attention against the one-thread-per-score kernels (a head size
+that the tiles do not take: 512 values and 8 zeros, which change no sum), the 128-row FP8 GEMM against the 32-row
+one, the grouping of routings against a call per piece."""
 import numpy as np
 import pytest
 
+import cases
 from _gpu import bits, cuda_moe, cuda_qgemm, lib
 from _oracle import P
 from apus_b200 import synth
 
 pytestmark = pytest.mark.gpu
+D, PAD = 512, 520
+
+
+def attn(c, q, ka, kb, s, h, d, idxw, bf16):
+    if not bf16:
+        o = np.empty((s, h, d), np.float32)
+        assert lib().apus_cuda_sparse_attn(P(q), P(c["sink"]), h, d, P(c["idx"]), idxw, s, D ** -0.5, P(ka), len(ka), P(kb), len(kb),
+                                           P(o)) == 0, lib().apus_cuda_last_error()
+        return o
+    import torch
+    lib()
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()   # noqa: E731
+    # a query pointer that is only 4-byte aligned is a legal one
+    qd = torch.empty(q.size + 1, device="cuda")[1:]
+    qd.copy_(t(q).reshape(-1))
+    sink, idx, a, b = t(c["sink"]), t(c["idx"]), t(synth.bf16_bits(ka).view(np.int16)), t(synth.bf16_bits(kb).view(np.int16))
+    o = torch.empty(s * h * d + 1, device="cuda")[1:]
+    assert lib().apus_cuda_sparse_attn_dev(qd.data_ptr(), sink.data_ptr(), h, d, idx.data_ptr(), idxw, s, D ** -0.5, a.data_ptr(),
+                                           len(ka), b.data_ptr(), len(kb), o.data_ptr(),
+                                           torch.cuda.current_stream().cuda_stream) == 0, lib().apus_cuda_last_error()
+    torch.cuda.synchronize()
+    return o.cpu().numpy().reshape(s, h, d)
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("values", ["bf16", "f32", "tiny", "sharp"])
+@pytest.mark.parametrize("s,h,idxw", [(1, 64, 1), (1, 64, 9), (2, 3, 129), (5, 64, 640), (7, 64, 911), (13, 64, 33), (32, 64, 130),
+                                      (33, 64, 257), (48, 20, 640), (2, 64, 1537)])
+def test_attention_tiles(s, h, idxw, values, bf16):
+    c = cases.sparse_attn_case(1000 * s + idxw, s, h, D, 40, 90, idxw, "holes" if s > 1 else "full")
+    rng = np.random.default_rng(idxw)
+    q, ka, kb = c["q"], c["kv_a"], c["kv_b"]
+    if values == "f32":                          # products that are not exact in f32
+        q = (q * np.float32(1.0009765625 + 2.0 ** -20)).astype(np.float32)
+    elif values == "tiny":                       # products below the normal range, in a few chunks of a few rows
+        q[:, :, 40:60] = synth.bf16_round((rng.standard_normal((s, h, 20)) * 2.0 ** -75).astype(np.float32))
+        ka[3, 40:60] = synth.bf16_round((rng.standard_normal(20) * 2.0 ** -70).astype(np.float32))
+    elif values == "sharp":                      # probabilities from 1 down to far below 2^-60
+        q = synth.bf16_round(q * np.float32(40.0))
+    got = attn(c, q, ka, kb, s, h, D, idxw, bf16)
+    wide = lambda a: np.concatenate([a, np.zeros(a.shape[:-1] + (PAD - D,), np.float32)], -1)   # noqa: E731
+    want = attn(c, wide(q), wide(ka), wide(kb), s, h, PAD, idxw, bf16)[:, :, :D]
+    assert np.array_equal(bits(got), bits(want))
 
 
 @pytest.mark.parametrize("M,O,K", [(64, 128, 128), (65, 256, 384), (127, 128, 1024), (129, 384, 256), (260, 4096, 640),

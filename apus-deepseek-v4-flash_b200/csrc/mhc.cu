@@ -47,11 +47,23 @@ mhc_mix_kernel(const float *__restrict__ x4, const float *__restrict__ fn, int n
     float acc = 0.f;
     if (j < nmix) {
         const float *f = fn + (size_t)j * nx;
-        for (int i = threadIdx.x * 4; i < nx; i += blockDim.x * 4) {
-            float4 a = __ldg(reinterpret_cast<const float4 *>(f + i));
-            float4 b = *reinterpret_cast<const float4 *>(x + i);
-            acc = fmaf(a.x, b.x, acc); acc = fmaf(a.y, b.y, acc);
-            acc = fmaf(a.z, b.z, acc); acc = fmaf(a.w, b.w, acc);
+        // the loads of eight steps are issued before the sums that use them: the kernel is a chain of L2 latencies
+        for (int i0 = threadIdx.x * 4; i0 < nx; i0 += blockDim.x * 32) {
+            float4 a[8], b[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int i = i0 + u * blockDim.x * 4;
+                if (i < nx) {
+                    a[u] = __ldg(reinterpret_cast<const float4 *>(f + i));
+                    b[u] = *reinterpret_cast<const float4 *>(x + i);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (i0 + u * blockDim.x * 4 < nx) {
+                    acc = fmaf(a[u].x, b[u].x, acc); acc = fmaf(a[u].y, b[u].y, acc);
+                    acc = fmaf(a[u].z, b[u].z, acc); acc = fmaf(a[u].w, b[u].w, acc);
+                }
         }
     } else {
         for (int i = threadIdx.x * 4; i < nx; i += blockDim.x * 4) {

@@ -421,7 +421,8 @@ int gemm_tc_status(int reset) {
     const int v8 = gemm_tc8_status(reset);          // the FP8 kernel keeps its own word (codes 11..15)
     const int vb = gemm_tcbf_status(reset);         // and the BF16 kernel (codes 21..23)
     const int va = attn_status(reset);              // and P.V of the sparse attention (31)
-    return v ? v : (v8 ? v8 : vb ? vb : va);
+    const int vl = linear_status(reset);            // and the chain linears (41, 42)
+    return v ? v : (v8 ? v8 : vb ? vb : va ? va : vl);
 }
 
 }  // namespace apus

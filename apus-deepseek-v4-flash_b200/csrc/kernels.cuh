@@ -153,6 +153,7 @@ struct LinCodes {
     float *s;
     int written;
 };
+int linear_status(int reset);             // status word of the bounded waits in the f32 linears (0 = none expired)
 int f32_linear_batched(const void *w, long long w_stride, const float *x, long long x_stride, int x_ld,
                        float *out, long long out_stride, int out_ld, int batch, int M, int K, int O,
                        int flags, cudaStream_t st, LinCodes *codes = nullptr);

@@ -110,3 +110,21 @@ def test_topk_selection(n, k, values):
     assert lib().apus_cuda_topk_stable(P(sc), n, k, P(idx), rows) == 0, lib().apus_cuda_last_error()
     want = np.argsort(-(sc + np.float32(0)).astype(np.float64), axis=1, kind="stable")[:, :k]
     assert np.array_equal(idx, want)
+
+
+@pytest.mark.parametrize("M,K,O", [(1, 8, 1), (1, 4096, 256), (2, 136, 33), (5, 264, 31), (8, 128, 1024), (17, 24, 5), (33, 520, 64),
+                                   (40, 392, 4400), (300, 256, 96), (700, 136, 1000)])
+def test_f32_linear_is_the_sequential_sum(M, K, O):
+    """Every layout of the f32 linears (one chain per lane, four tokens per lane, two rows per lane; short K tiles,
+    ragged rows and tokens): products and sums rounded one by one, k ascending."""
+    rng = np.random.default_rng(M + O)
+    w = rng.standard_normal((O, K)).astype(np.float32)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    x[0, ::3] = -0.0
+    want = np.zeros((M, O), np.float32)
+    for k in range(K):
+        want += x[:, k, None] * w[None, :, k]
+    got = np.empty((M, O), np.float32)
+    assert lib().apus_cuda_f32_linear(P(w), P(x), P(got), M, K, O, 0) == 0, lib().apus_cuda_last_error()
+    lib().apus_cuda_forget(P(w))
+    assert np.array_equal(bits(got), bits(want))

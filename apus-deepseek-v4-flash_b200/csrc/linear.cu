@@ -2,9 +2,10 @@
 // head weights, grouped o-projection and the LM head (reference
 // c/attn.h:460-666, c/attn.h:1439-1492, c/model.h:528-647).
 //
-// Two kernels: `f32_linear_seq_kernel` keeps the reference's summation order
-// (the default, see apus_cuda_set_sum_order) and `f32_linear_kernel` is the
-// split-K variant of the tree order, described here:
+// `f32_linear_seq_kernel` and, for few tokens on f32 weights, `f32_chain_kernel`
+// keep the reference's summation order (the default, see
+// apus_cuda_set_sum_order); `f32_linear_kernel` is the split-K variant of the
+// tree order, described here:
 // out[m,o] = sum_k x[m,k] * w[o,k] in f32.  A CTA of 8 warps owns OT output rows
 // and up to MT activation rows; the warps split K into eight contiguous ranges,
 // every lane keeps OT*MT partial sums, and the partials are combined by a

@@ -270,11 +270,13 @@ gemm_tc8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
 //   warp 8      TMA producer (weight tile + activation tile per 128-wide block of K)
 //   warp 9      MMA issuer, four accumulators of 128 TMEM columns; owns the allocation
 //   warp 10     scales: per block the 128 products as[m, kb] * 2^(ws[kb] - 127), once for the whole tile
-// The fold of a block is dot * s added to the running sum, s the scale product.  s is a power of two, so with
+// The fold of a block is dot * s added to the running sum, s the scale product.  Where s is a power of two with
 // 2^-100 <= s <= 2^90 (or s = 0, a row past the end) the multiplication is exact: dots are multiples of 2^-18
 // below 2^25.  One fused multiply-add then gives the sum the separate multiply and add give, and two of them go
-// into one instruction (f32x2): 32 instructions per thread and block where there were 384.  The scale warp
-// looks at every product; a block with one outside the window takes the two-instruction fold.
+// into one instruction (f32x2): 32 instructions per thread and block where there were 384.  Weight scales are
+// powers of two by their format and act_quant makes such activation scales, but apus_cuda_fp8_gemm takes the
+// caller's, which can be any f32.  The scale warp looks at every product; a block with one that is no power of
+// two or lies outside the window takes the two-instruction fold.
 // Bound by the tiles' way from L2: 32 KB per block, 128 flop per byte.  B200, 4096^3: 219 -> 151 us, 910 TFLOP/s.
 constexpr int T8W_N = 128, T8W_NS = 6, T8W_NACC = 4, T8W_THREADS = 352;
 constexpr int T8W_STAGE = T8_A_BYTES + T8W_N * 128;
@@ -384,7 +386,8 @@ gemm_tc8_wide_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
                     as[j] = __fmul_rn(as[j], ws);
-                    ok = ok && (as[j] == 0.f || (as[j] >= 7.88860905e-31f && as[j] <= 1.23794004e27f));     // 2^-100, 2^90
+                    const bool pow2 = (__float_as_uint(as[j]) & 0x7fffffu) == 0u;
+                    ok = ok && (as[j] == 0.f || (pow2 && as[j] >= 7.88860905e-31f && as[j] <= 1.23794004e27f));     // 2^-100, 2^90
                 }
                 *reinterpret_cast<float4 *>(s_sw + b * T8W_N + 4 * lane) = make_float4(as[0], as[1], as[2], as[3]);
                 const int all = __all_sync(0xffffffffu, ok);

@@ -1,8 +1,9 @@
 // Stable top-k selection and index-gathered sparse attention.
-#include <map>
+#include <mutex>
+#include <thread>
+#include <vector>
 #include <cooperative_groups.h>
-#include "common.cuh"
-#include "kernels.cuh"
+#include "runtime.cuh"
 #include "tc_common.cuh"
 
 namespace apus {
@@ -1045,22 +1046,69 @@ __global__ void compact_ids_kernel(const int32_t *__restrict__ idxs, int idxw,
     if (tid == 0) { ns[t] = s_base; bad[t] = 0; }
 }
 
-// Scores / compacted ids between the kernels of a call: the caller's scratch (a model
-// object keeps its own), else one buffer of the library, which only grows.
-static void *g_scratch = nullptr;
-static size_t g_scratch_cap = 0;
-static void *ensure_scratch(size_t bytes) {
-    if (bytes <= g_scratch_cap) return g_scratch;
-    if (g_scratch) { cudaDeviceSynchronize(); cudaFree(g_scratch); }
-    g_scratch = nullptr; g_scratch_cap = 0;
-    if (cudaMalloc(&g_scratch, bytes) != cudaSuccess) {
-        set_error("sparse_attn: scratch of %zu bytes", bytes);
-        g_scratch = nullptr;
-        return nullptr;
-    }
-    g_scratch_cap = bytes;
-    return g_scratch;
+// Scores / compacted ids between the kernels of a call: the caller's scratch (a model object keeps its own), else a
+// buffer of the library that belongs to the call's stream.  Calls on several streams never share one (a shared one
+// would let a call read the ids another is writing, or take the walk flags of another's rows); a call holds the lock
+// until its last launch, so that those of two threads on one stream do not mix and none loses its buffer to a growing
+// one.  A call that is being recorded gets memory that its graph owns.  At most SCR_MAX buffers are kept, the longest
+// unused one makes room for a new stream's, apus_cuda_disable frees them all.
+#define SCR_MAX 16
+struct ScrSlot {
+    int dev;
+    cudaStream_t st;
+    std::thread::id th;                                    // cudaStreamPerThread is another stream in every thread
+    DevBuf buf;
+    unsigned long long used;
+};
+static std::mutex g_scr_mu;
+static std::vector<ScrSlot> g_scr;
+static unsigned long long g_scr_calls = 0;
+static void scr_release() {
+    std::lock_guard<std::mutex> lock(g_scr_mu);
+    for (ScrSlot &s : g_scr) s.buf.release();
+    g_scr.clear();
 }
+struct ScrReg { ScrReg() { on_disable(scr_release, nullptr); } };
+static ScrReg g_scr_reg;
+
+struct CallScratch {
+    std::unique_lock<std::mutex> lock;
+    cudaStream_t st;
+    void *p = nullptr;
+    bool recorded = false;
+    explicit CallScratch(cudaStream_t s) : st(s) {}
+    ~CallScratch() { if (recorded && p) cudaFreeAsync(p, st); }
+    CallScratch(const CallScratch &) = delete;
+    CallScratch &operator=(const CallScratch &) = delete;
+    int get(size_t bytes) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        APUS_CUDA_OK(cudaStreamIsCapturing(st, &cs));
+        if (cs != cudaStreamCaptureStatusNone) {
+            recorded = true;
+            APUS_CUDA_OK(cudaMallocAsync(&p, bytes, st));
+            return 0;
+        }
+        int dev = 0;
+        APUS_CUDA_OK(cudaGetDevice(&dev));
+        const std::thread::id th = st == cudaStreamPerThread ? std::this_thread::get_id() : std::thread::id();
+        lock = std::unique_lock<std::mutex>(g_scr_mu);
+        ScrSlot *slot = nullptr, *idle = nullptr;
+        for (ScrSlot &s : g_scr) {
+            if (s.dev == dev && s.st == st && s.th == th) slot = &s;
+            if (s.dev == dev && (!idle || s.used < idle->used)) idle = &s;
+        }
+        if (!slot && (g_scr.size() < SCR_MAX || !idle)) {
+            g_scr.push_back(ScrSlot{dev, st, th, DevBuf(), 0});
+            slot = &g_scr.back();
+        } else if (!slot) {
+            APUS_CUDA_OK(cudaDeviceSynchronize());         // another stream may still be using it
+            slot = idle;
+            slot->st = st; slot->th = th;
+        }
+        slot->used = ++g_scr_calls;
+        return slot->buf.get(bytes, &p);
+    }
+};
 // Layout of that scratch: scores, compacted ids, their counts, denominators, the walk flags of P.V.
 struct SaScratch {
     size_t ids, ns, den, bad, bytes;
@@ -1174,8 +1222,9 @@ int sparse_attn(const float *q, const float *sink, int h, int d,
     if (s <= 0 || idxw <= 0) return 0;
     const SaScratch lay(h, idxw, s);
     APUS_REQUIRE(!callers || lay.bytes <= callers_cap, "sparse_attn: scratch of %zu bytes given, %zu needed", callers_cap, lay.bytes);
-    char *scratch = (char *)(callers ? callers : ensure_scratch(lay.bytes));
-    if (!scratch) return 1;
+    CallScratch own(st);
+    if (!callers && own.get(lay.bytes)) return 1;
+    char *scratch = (char *)(callers ? callers : own.p);
     float *sc = (float *)scratch;
     int32_t *ids = (int32_t *)(scratch + lay.ids);
     int *ns = (int *)(scratch + lay.ns);

@@ -67,7 +67,11 @@ int DevQW::table_for(int M, bool pair, const DevQW *other, GemmGroup **out, int 
         }
         GemmGroup *d = nullptr;
         APUS_CUDA_OK(cudaMalloc(&d, n * sizeof(GemmGroup)));
-        APUS_CUDA_OK(cudaMemcpy(d, h.data(), n * sizeof(GemmGroup), cudaMemcpyHostToDevice));
+        if (upload_now(d, h.data(), n * sizeof(GemmGroup))) {
+            set_error("upload of a work-item table failed");
+            cudaFree(d);
+            return 1;
+        }
         it = tables.emplace(key, d).first;
     }
     *out = it->second;
@@ -137,6 +141,16 @@ int branch_end(int i, cudaStream_t main) {
 }
 
 // ---- uploads ----------------------------------------------------------------------------------
+// Both are complete when they return.  cudaMemcpy may come back with a pageable source only staged and a device source
+// only queued, cudaMemset with its store queued, on the default stream -- which the library's own streams, being
+// non-blocking, do not wait for: a kernel launched right after could read old bytes, or have its result cleared.
+int upload_now(void *dst, const void *src, size_t bytes) {
+    return cudaMemcpy(dst, src, bytes, cudaMemcpyDefault) == cudaSuccess && cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess ? 0 : 1;
+}
+int clear_now(void *dst, size_t bytes) {
+    return cudaMemset(dst, 0, bytes) == cudaSuccess && cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess ? 0 : 1;
+}
+
 int upload_qw(int fmt, const uint8_t *codes, const uint8_t *scales, int O, int K,
               uint8_t *dst_codes, uint8_t *dst_scales, int *zero_scale) {
     Ctx &c = ctx();
@@ -186,11 +200,11 @@ DevQW *new_qw(int fmt, const uint8_t *codes, const uint8_t *scales, int O, int K
         // tcgen05 kernel: no re-tiling; a device buffer of the caller is used in place
         const bool adopt = is_device_ptr(codes) && ((uintptr_t)codes & 15) == 0;
         bool ok = cudaMalloc(&w->scales, sb) == cudaSuccess &&
-                  cudaMemcpy(w->scales, scales, sb, cudaMemcpyDefault) == cudaSuccess;
+                  upload_now(w->scales, scales, sb) == 0;
         if (ok && adopt) { w->codes = const_cast<uint8_t *>(codes); w->owned = false; }
         else if (ok) {
             ok = cudaMalloc(&w->codes, cb) == cudaSuccess &&
-                 cudaMemcpy(w->codes, codes, cb, cudaMemcpyDefault) == cudaSuccess;
+                 upload_now(w->codes, codes, cb) == 0;
             if (ok) ctx().bytes_uploaded += cb + sb;
         }
         if (!ok) set_error("upload of %zu FP8 weight bytes failed", cb + sb);
@@ -241,7 +255,7 @@ const void *cached_dense(const void *host, size_t bytes) {
     if (it != c.dcache.end() && it->second->cap >= bytes) return it->second->p;
     DevBuf *b = it != c.dcache.end() ? it->second : new DevBuf();
     if (b->get(bytes, nullptr)) return nullptr;
-    if (cudaMemcpy(b->p, host, bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (upload_now(b->p, host, bytes)) {
         set_error("upload of %zu dense weight bytes failed", bytes);
         return nullptr;
     }
@@ -391,7 +405,7 @@ int stream_scratch(cudaStream_t st, size_t bytes, void **ws, size_t n_counters, 
         cudaStreamIsCapturing(st, &cs);
         APUS_REQUIRE(cs == cudaStreamCaptureStatusNone, "stream counters would have to grow inside a stream capture");
         if (s.cnt.get(cb < 4096 ? 4096 : 2 * cb, nullptr)) return 1;
-        APUS_CUDA_OK(cudaMemset(s.cnt.p, 0, s.cnt.cap));
+        APUS_REQUIRE(clear_now(s.cnt.p, s.cnt.cap) == 0, "stream counters could not be cleared");
     }
     if (ws) *ws = s.ws.p;
     if (counters) *counters = s.cnt.as<int>();

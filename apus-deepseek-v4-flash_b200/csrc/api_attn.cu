@@ -36,7 +36,7 @@ const void *get_dense(WeightOwner *own, const void *src, size_t bytes) {
     if (!own) return cached_dense(src, bytes);
     if (is_device_ptr(src)) return src;           // used in place; the caller keeps it alive
     DevBuf *b = new DevBuf();
-    if (b->get(bytes, nullptr) || cudaMemcpy(b->p, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (b->get(bytes, nullptr) || upload_now(b->p, src, bytes)) {
         set_error("upload of %zu dense weight bytes failed", bytes);
         b->release(); delete b;
         return nullptr;

@@ -127,7 +127,7 @@ const float *rope_rows_dev(const float *cos, const float *sin, int rows, int hal
     }
     DevBuf *b = it != cache.end() ? it->second : new DevBuf();
     if (b->get(cs.size() * 4, nullptr)) return nullptr;
-    if (cudaMemcpy(b->p, cs.data(), cs.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
+    if (upload_now(b->p, cs.data(), cs.size() * 4)) return nullptr;
     cache[cos] = b;
     return b->as<float>();
 }

@@ -84,7 +84,7 @@ int ApusCudaMoe::ensure(int s, int n_rout) {
             b_hs.get(R * (inter / 128) * 4, nullptr) || b_eo.get(R * dim * 4, nullptr) ||
             b_t13.get(max_groups * sizeof(TcGroup), nullptr) || b_t2.get(max_groups * sizeof(TcGroup), nullptr))
             return 1;
-        APUS_CUDA_OK(cudaMemset(b_ng.p, 0, 256));
+        APUS_REQUIRE(clear_now(b_ng.p, 256) == 0, "moe: the work-item counters could not be cleared");
         if (use_tc && (tc_make_act_map(map_xq, b_xq.p, (long long)(b_xq.cap / dim), dim) ||
                        tc_make_act_map(map_hq, b_hq.p, (long long)(b_hq.cap / inter), inter) ||
                        tc_make_act_map(map_xq64, b_xq.p, (long long)(b_xq.cap / dim), dim, 64) ||
@@ -301,10 +301,10 @@ ApusCudaMoe *apus_cuda_moe_create(const ApusMoeW *w, int e_lo, int e_hi) {
     const size_t total = (size_t)nl * (2 * (c13 + s13) + c2 + s2);
     bool ok = true;
     ok = ok && cudaMalloc(&m->gate_w, (size_t)w->E * w->dim * 4) == cudaSuccess;
-    ok = ok && cudaMemcpy(m->gate_w, w->gate_w, (size_t)w->E * w->dim * 4, cudaMemcpyDefault) == cudaSuccess;
+    ok = ok && upload_now(m->gate_w, w->gate_w, (size_t)w->E * w->dim * 4) == 0;
     if (ok && !w->hash) {
         ok = ok && cudaMalloc(&m->gate_bias, (size_t)w->E * 4) == cudaSuccess;
-        ok = ok && cudaMemcpy(m->gate_bias, w->gate_bias, (size_t)w->E * 4, cudaMemcpyDefault) == cudaSuccess;
+        ok = ok && upload_now(m->gate_bias, w->gate_bias, (size_t)w->E * 4) == 0;
     }
     if (!ok) { set_error("moe_create: upload of the gate failed"); apus_cuda_moe_destroy(m); return nullptr; }
     m->sl.code_stride13 = c13; m->sl.scale_stride13 = s13;
@@ -346,12 +346,12 @@ ApusCudaMoe *apus_cuda_moe_create(const ApusMoeW *w, int e_lo, int e_hi) {
         uint8_t *e2 = q;
         m->rw1 = d1; m->rw3 = d3; m->rw2 = d2; m->rs1 = e1; m->rs3 = e3; m->rs2 = e2;
         for (int le = 0; le < nl; le++) {
-            bool ok2 = cudaMemcpy(d1 + le * c13, r1[le].packed, c13, cudaMemcpyDefault) == cudaSuccess &&
-                       cudaMemcpy(d3 + le * c13, r3[le].packed, c13, cudaMemcpyDefault) == cudaSuccess &&
-                       cudaMemcpy(d2 + le * c2, r2[le].packed, c2, cudaMemcpyDefault) == cudaSuccess &&
-                       cudaMemcpy(e1 + le * s13, r1[le].scales, s13, cudaMemcpyDefault) == cudaSuccess &&
-                       cudaMemcpy(e3 + le * s13, r3[le].scales, s13, cudaMemcpyDefault) == cudaSuccess &&
-                       cudaMemcpy(e2 + le * s2, r2[le].scales, s2, cudaMemcpyDefault) == cudaSuccess;
+            bool ok2 = upload_now(d1 + le * c13, r1[le].packed, c13) == 0 &&
+                       upload_now(d3 + le * c13, r3[le].packed, c13) == 0 &&
+                       upload_now(d2 + le * c2, r2[le].packed, c2) == 0 &&
+                       upload_now(e1 + le * s13, r1[le].scales, s13) == 0 &&
+                       upload_now(e3 + le * s13, r3[le].scales, s13) == 0 &&
+                       upload_now(e2 + le * s2, r2[le].scales, s2) == 0;
             if (!ok2) { set_error("moe_create: upload of expert %d failed", e_lo + le); apus_cuda_moe_destroy(m); return nullptr; }
         }
         c.bytes_uploaded += total;
@@ -476,7 +476,7 @@ int apus_cuda_moe_set_hash_table(ApusCudaMoe *m, const int64_t *tid2eid, int64_t
     if (m->tid2eid) { cudaDeviceSynchronize(); cudaFree(m->tid2eid); m->tid2eid = nullptr; }
     size_t bytes = (size_t)vocab * m->topk * 8;
     APUS_CUDA_OK(cudaMalloc(&m->tid2eid, bytes));
-    APUS_CUDA_OK(cudaMemcpy(m->tid2eid, tid2eid, bytes, cudaMemcpyDefault));
+    APUS_REQUIRE(upload_now(m->tid2eid, tid2eid, bytes) == 0, "set_hash_table: upload of %zu bytes failed", bytes);
     m->vocab = vocab;
     return 0;
 }

@@ -80,6 +80,9 @@ int branch_end(int i, cudaStream_t main);
 // apus_cuda_forget).
 void on_disable(void (*release_all)(), void (*forget_one)(const void *));
 
+// Memory to the device / device memory to zero, complete when the call returns (load-time copies; nonzero on failure).
+int upload_now(void *dst, const void *src, size_t bytes);
+int clear_now(void *dst, size_t bytes);
 // Upload + re-tile one quantised matrix (host pointers in `codes`/`scales`).
 int upload_qw(int fmt, const uint8_t *codes, const uint8_t *scales, int O, int K,
               uint8_t *dst_codes, uint8_t *dst_scales, int *zero_scale);

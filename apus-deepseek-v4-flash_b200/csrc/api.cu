@@ -1,6 +1,7 @@
 // C ABI, part 1: lifecycle, weight cache, kernel-level host-pointer entry points
 // and the single-matrix device-resident entry points (include/apus_b200.h).
 #include <stdarg.h>
+#include <atomic>
 #include <tuple>
 #include <stdlib.h>
 
@@ -17,6 +18,34 @@ void set_error(const char *fmt, ...) {
     va_start(ap, fmt);
     vsnprintf(t_err, sizeof t_err, fmt, ap);
     va_end(ap);
+}
+
+// ---- bounded waits -----------------------------------------------------------------------
+__device__ int g_wait_word = 0;
+int *wait_word() {
+    static std::atomic<int *> at[64];              // by device
+    int dev = 0;
+    void *p = nullptr;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
+        p = at[dev].load();
+        if (!p && cudaGetSymbolAddress(&p, g_wait_word) == cudaSuccess) at[dev].store(static_cast<int *>(p));
+    }
+    if (!p) set_error("the status word of the bounded waits has no address on device %d", dev);
+    return static_cast<int *>(p);
+}
+int wait_status(int reset) {
+    int v = 0;
+    if (cudaMemcpyFromSymbol(&v, g_wait_word, sizeof(int)) != cudaSuccess) return -1;
+    if (reset && v) {
+        const int z = 0;
+        cudaMemcpyToSymbol(g_wait_word, &z, sizeof(int));
+    }
+    return v;
+}
+int wait_check(const char *what) {
+    const int v = wait_status(1);
+    APUS_REQUIRE(v == 0, "%s: a bounded wait ran out inside a kernel (code %d)", what, v);
+    return 0;
 }
 
 // ---- device buffers ------------------------------------------------------------------
@@ -103,6 +132,7 @@ int ensure_enabled() {
                   prop.major, prop.minor);
         return 1;
     }
+    if (!wait_word()) return 1;
     APUS_CUDA_OK(cudaStreamCreateWithFlags(&c.own_stream, cudaStreamNonBlocking));
     c.stream = c.own_stream;
     for (int i = 0; i < Ctx::N_AUX; i++) {
@@ -579,11 +609,7 @@ static int host_qlinear(int fmt, const uint8_t *codes, const uint8_t *scales, in
         return 1;
     APUS_CUDA_OK(cudaMemcpyAsync(out, dout, (size_t)M * O * 4, cudaMemcpyDeviceToHost, c.stream));
     APUS_CUDA_OK(cudaStreamSynchronize(c.stream));
-    if (w->tc) {
-        int stt = gemm_tc_status(1);
-        APUS_REQUIRE(stt == 0, "a bounded wait expired inside a tcgen05 kernel (code %d)", stt);
-    }
-    return 0;
+    return w->tc ? wait_check("linear") : 0;
 }
 
 int apus_cuda_fp8_linear(const ApusFp8W *w, const float *x, float *out, int M, int K, int O) {
@@ -632,9 +658,7 @@ static int host_qgemm(int fmt, const uint8_t *w, const uint8_t *ws, const uint8_
     if (qgemm_dev(dw, nullptr, (uint8_t *)dq, (float *)ds, M, (float *)dout, false, 0.f, c.stream)) return 1;
     APUS_CUDA_OK(cudaMemcpyAsync(out, dout, (size_t)M * O * 4, cudaMemcpyDeviceToHost, c.stream));
     APUS_CUDA_OK(cudaStreamSynchronize(c.stream));
-    int stt = gemm_tc_status(1);
-    APUS_REQUIRE(stt == 0, "a bounded wait expired inside a tcgen05 kernel (code %d)", stt);
-    return 0;
+    return wait_check("gemm");
 }
 
 int apus_cuda_fp8_gemm(const uint8_t *w, const uint8_t *ws, const uint8_t *acodes,
@@ -675,12 +699,11 @@ int apus_cuda_fp4_gemm_tc(const uint8_t *w, const uint8_t *ws, const uint8_t *ac
     a.scales_a = (const uint8_t *)ds; a.ascales = (const float *)das;
     a.groups = (const TcGroup *)dg; a.n_groups = ng; a.O = O; a.K = K; a.pair = 0; a.round_out = 0;
     a.out = (float *)dout;
-    gemm_tc_status(1);
+    wait_status(1);
     if (gemm_tc(a, c.stream)) return 1;
     APUS_CUDA_OK(cudaMemcpyAsync(out, dout, (size_t)M * O * 4, cudaMemcpyDeviceToHost, c.stream));
     APUS_CUDA_OK(cudaStreamSynchronize(c.stream));
-    int stt = gemm_tc_status(1);
-    APUS_REQUIRE(stt == 0, "fp4_gemm_tc: a bounded wait expired inside the kernel (code %d)", stt);
+    if (wait_check("fp4_gemm_tc")) return 1;
     return 0;
 }
 

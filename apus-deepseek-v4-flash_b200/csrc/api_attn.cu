@@ -540,8 +540,7 @@ int apus_cuda_attention(const ApusAttnCfg *cfg, const ApusAttnW *w, ApusAttnS *s
         APUS_CUDA_OK(cudaStreamSynchronize(sm));
         attn_state_commit(*cfg, st, g_state);
         if (ratio && interm) { interm->comp_nb = st->comp.nb - nb0; interm->idx_nb = cfg->has_indexer ? st->idx_comp.nb - inb0 : 0; }
-        int stt = gemm_tc_status(1);
-        APUS_REQUIRE(stt == 0, "attention: a bounded wait expired inside a tcgen05 kernel (code %d)", stt);
+        if (wait_check("attention")) return 1;
         return 0;
     }
     // rope rows: per token [cos | sin] at its position and at the first position of the block it completes
@@ -590,8 +589,7 @@ int apus_cuda_attention(const ApusAttnCfg *cfg, const ApusAttnW *w, ApusAttnS *s
     if (ratio) {
         if (interm) { interm->comp_nb = st->comp.nb - nb0; interm->idx_nb = cfg->has_indexer ? st->idx_comp.nb - inb0 : 0; }
     }
-    int stt = gemm_tc_status(1);
-    APUS_REQUIRE(stt == 0, "attention: a bounded wait expired inside a tcgen05 kernel (code %d)", stt);
+    if (wait_check("attention")) return 1;
     return 0;
 }
 

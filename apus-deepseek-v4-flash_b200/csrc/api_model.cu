@@ -713,8 +713,7 @@ int apus_cuda_block_forward_v(const ApusCudaLayerDesc *d, int hc, int iters, flo
         if (attn_state_download(c, st, S, sm)) return 1;
         APUS_CUDA_OK(cudaStreamSynchronize(sm));
         attn_state_commit(c, st, S);
-        int stt2 = gemm_tc_status(1);
-        APUS_REQUIRE(stt2 == 0, "block_forward: a bounded wait expired inside a tcgen05 kernel (code %d)", stt2);
+        if (wait_check("block_forward")) return 1;
         return 0;
     }
     if (attn_step_bufs(c, max_nb, 1, ws, &sb)) return 1;
@@ -739,8 +738,7 @@ int apus_cuda_block_forward_v(const ApusCudaLayerDesc *d, int hc, int iters, flo
     if (attn_state_download(c, st, S, sm)) return 1;
     APUS_CUDA_OK(cudaStreamSynchronize(sm));
     attn_state_commit(c, st, S);
-    int stt = gemm_tc_status(1);
-    APUS_REQUIRE(stt == 0, "block_forward: a bounded wait expired inside a tcgen05 kernel (code %d)", stt);
+    if (wait_check("block_forward")) return 1;
     return 0;
 }
 
@@ -875,8 +873,7 @@ int apus_cuda_model_forward_group(ApusCudaModel *const *ms, int n, const int64_t
             APUS_CUDA_OK(cudaMemcpyAsync(next[i], m->tok.p, (size_t)m->B * 4, cudaMemcpyDeviceToHost, mstream(m)));
     }
     if (group_sync(ms, n)) return 1;
-    int stt = gemm_tc_status(1);
-    APUS_REQUIRE(stt == 0, "model_forward: a bounded wait expired inside a tcgen05 kernel (code %d)", stt);
+    if (wait_check("model_forward")) return 1;
     return 0;
 }
 
@@ -943,8 +940,7 @@ static int forward_ex(ApusCudaModel *m, const int64_t *ids, int s, float *logits
         if (next) APUS_CUDA_OK(cudaMemcpyAsync(next, m->tok.p, B * 4, cudaMemcpyDeviceToHost, st));
     }
     APUS_CUDA_OK(cudaStreamSynchronize(st));
-    int stt = gemm_tc_status(1);
-    APUS_REQUIRE(stt == 0, "%s: a bounded wait expired inside a tcgen05 kernel (code %d)", what, stt);
+    if (wait_check(what)) return 1;
     return 0;
 }
 
@@ -984,8 +980,7 @@ int apus_cuda_model_forward_all(ApusCudaModel *m, const int64_t *ids, int s, flo
             APUS_CUDA_OK(cudaMemcpy2DAsync(next_all + t, (size_t)s * 4, m->tok.p, 4, 4, B, cudaMemcpyDeviceToHost, st));
     }
     APUS_CUDA_OK(cudaStreamSynchronize(st));
-    int stt = gemm_tc_status(1);
-    APUS_REQUIRE(stt == 0, "model_forward: a bounded wait expired inside a tcgen05 kernel (code %d)", stt);
+    if (wait_check("model_forward")) return 1;
     return 0;
 }
 
@@ -1045,8 +1040,7 @@ int apus_cuda_model_generate_group(ApusCudaModel *const *ms, int n, const int64_
     if (ms_decode) *ms_decode = b;
     cudaEventDestroy(e0); cudaEventDestroy(e1); cudaEventDestroy(e2);
     for (int i = 0; i < n; i++) cudaEventDestroy(tmp[i]);
-    int stt = gemm_tc_status(1);
-    APUS_REQUIRE(stt == 0, "model_generate: a bounded wait expired inside a tcgen05 kernel (code %d)", stt);
+    if (wait_check("model_generate")) return 1;
     return 0;
 }
 
@@ -1324,8 +1318,7 @@ int apus_cuda_mtp_forward(ApusCudaMtp *mt, const float *h_in, const int64_t *ids
     if (next) APUS_CUDA_OK(cudaMemcpyAsync(next, mt->tok.p, B * 4, cudaMemcpyDeviceToHost, st));
     if (h_last) APUS_CUDA_OK(cudaMemcpyAsync(h_last, mt->hlast.p, B * hd * 4, cudaMemcpyDeviceToHost, st));
     APUS_CUDA_OK(cudaStreamSynchronize(st));
-    int stt = gemm_tc_status(1);
-    APUS_REQUIRE(stt == 0, "mtp_forward: a bounded wait expired inside a tcgen05 kernel (code %d)", stt);
+    if (wait_check("mtp_forward")) return 1;
     return 0;
 }
 
@@ -1660,8 +1653,7 @@ int apus_cuda_dspark_draft_round(ApusCudaDspark *ds, int64_t anchor, const float
     if (ds_bufs(ds, 1)) return 1;
     APUS_CUDA_OK(cudaMemcpyAsync(ds->mh.p, mh_row, (size_t)ds->n_targets * m->dim * 4, cudaMemcpyHostToDevice, st));
     if (ds_round(ds, anchor, ds->mh.as<float>(), start_pos, drafts, confidence, logits_final, stage_h, st)) return 1;
-    int stt = gemm_tc_status(1);
-    APUS_REQUIRE(stt == 0, "dspark_draft_round: a bounded wait expired inside a tcgen05 kernel (code %d)", stt);
+    if (wait_check("dspark_draft_round")) return 1;
     return 0;
 }
 
@@ -1932,8 +1924,7 @@ int apus_cuda_model_read(ApusCudaModel *m, float *logits, int32_t *next) {
     if (logits) APUS_CUDA_OK(cudaMemcpyAsync(logits, m->logits.p, (size_t)m->B * m->vocab * 4, cudaMemcpyDeviceToHost, st));
     if (next) APUS_CUDA_OK(cudaMemcpyAsync(next, m->tok.p, (size_t)m->B * 4, cudaMemcpyDeviceToHost, st));
     APUS_CUDA_OK(cudaStreamSynchronize(st));
-    int stt = gemm_tc_status(1);
-    APUS_REQUIRE(stt == 0, "model: a bounded wait expired inside a tcgen05 kernel (code %d)", stt);
+    if (wait_check("model")) return 1;
     return 0;
 }
 

@@ -645,12 +645,11 @@ int apus_cuda_moe_forward(const ApusMoeW *w, const float *x, const int64_t *ids,
     }
     APUS_CUDA_OK(cudaStreamSynchronize(c.stream));
     if (m->use_tc) {
-        int stt = gemm_tc_status(1);
-        APUS_REQUIRE(stt == 0, "moe_forward: a bounded wait expired inside the tcgen05 kernel (code %d)", stt);
+        if (wait_check("moe_forward")) return 1;
     }
     return 0;
 }
 
-int apus_cuda_kernel_status(int reset) { return gemm_tc_status(reset); }
+int apus_cuda_kernel_status(int reset) { return wait_status(reset); }
 
 }  // extern "C"

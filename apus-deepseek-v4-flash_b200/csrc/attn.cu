@@ -805,7 +805,6 @@ sparse_pv_tile_kernel(const float *__restrict__ p, const float *__restrict__ den
 // banks), so that one 16-byte load gives the factor pairs of two heads.  Per candidate a thread issues HG / 2 + 1
 // shared loads for HG * NPAIR packed multiply-adds.
 #define PVS_NS 3
-__device__ int g_attn_status = 0;         // 31: a row copy did not arrive within the wait's budget
 template <bool BF16, int HG, int NPAIR, int T, int NT, bool BULK>
 struct PvCfg {
     static constexpr int ROWB = NT * NPAIR * (BF16 ? 4 : 8);     // bytes of a row's segment
@@ -875,7 +874,7 @@ __global__ void __launch_bounds__(NT)
 sparse_pv_stage_kernel(const float *__restrict__ p, const float *__restrict__ den, int h, int d,
                        const int32_t *__restrict__ ids, const int *__restrict__ ns, int idxw, const void *kv_a, int64_t na,
                        const void *kv_b, float *__restrict__ o, size_t a_stride, size_t b_stride, int seq_mod, const SaRope rope,
-                       const int *__restrict__ bad) {
+                       const int *__restrict__ bad, int *__restrict__ status) {
     APUS_PDL_WAIT();
     APUS_PDL_GO();
     using Cf = PvCfg<BF16, HG, NPAIR, T, NT, BULK>;
@@ -984,7 +983,7 @@ sparse_pv_stage_kernel(const float *__restrict__ p, const float *__restrict__ de
         id_store(c + 3, id_after);                             // slot of tile c - 1, whose copies are all issued
     }
     if (fail) {
-        if (tid == 0) atomicCAS(&g_attn_status, 0, 31);
+        if (tid == 0) atomicCAS(status, 0, 31);               // a row copy did not arrive in time
         for (int i = 0; i < 2000; i++) __nanosleep(1000);      // copies already issued to this CTA's shared memory land
         return;
     }
@@ -1122,16 +1121,6 @@ struct SaScratch {
 };
 size_t sparse_attn_scratch(int h, int idxw, int s) { return SaScratch(h, idxw, s).bytes; }
 
-int attn_status(int reset) {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_attn_status, sizeof(int)) != cudaSuccess) return -1;
-    if (reset && v) {
-        int z = 0;
-        cudaMemcpyToSymbol(g_attn_status, &z, sizeof(int));
-    }
-    return v;
-}
-
 // ---- launches of the tiled kernels ----
 template <bool BF16, int HL, int CL, int WH, int WC>
 static int scores_launch(const float *q, int h, int d, const int32_t *ids, const int *ns, int idxw, int s, float scale,
@@ -1151,9 +1140,10 @@ static int pv_launch(const float *sc, const float *den, int h, int d, const int3
                      size_t sb, int seq_mod, const SaRope &rope) {
     using Cf = PvCfg<BF16, HG, NPAIR, T, NT, BULK>;
     auto kern = sparse_pv_stage_kernel<BF16, HG, NPAIR, T, NT, BULK>;
-    if (ensure_dyn_smem((const void *)kern, Cf::SMEM + 64)) return 1;
+    int *status = wait_word();
+    if (!status || ensure_dyn_smem((const void *)kern, Cf::SMEM + 64)) return 1;
     launch_k(kern, dim3((unsigned)ceil_div(h, HG), (unsigned)s, (unsigned)(d / (2 * NPAIR * NT))), NT, Cf::SMEM, st,
-             sc, den, h, d, ids, ns, idxw, kv_a, na, kv_b, o, sa, sb, seq_mod, rope, bad);
+             sc, den, h, d, ids, ns, idxw, kv_a, na, kv_b, o, sa, sb, seq_mod, rope, bad, status);
     APUS_LAUNCHED();
     return 0;
 }

@@ -107,6 +107,14 @@ static inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 blo
         if (!(cond)) { apus::set_error(__VA_ARGS__); return 1; }               \
     } while (0)
 
+// ---- bounded waits -------------------------------------------------------------------------------
+// A wait on an mbarrier gives up after a while (mbar_wait, tc_common.cuh).  Its kernel then records a code in the one
+// word the current device has for them -- the first code stays --, leaves its outputs unwritten and returns.  1..6 are
+// of the MXFP4 GEMM, 11..16 of the FP8 ones, 21..24 of the BF16 ones, 31 of P.V, 41 and 42 of the chain linears.
+int *wait_word();                               // api.cu: address of that word (NULL + message on failure)
+int wait_status(int reset);                     // api.cu: its value, 0 = none ran out; one copy, on the default stream
+int wait_check(const char *what);               // api.cu: reads and clears it: nonzero + message naming `what` if one ran out
+
 // ---- scalar format helpers (device + host) -------------------------------------
 
 // acc + s[0] + s[1] + ... + s[n-1], one accumulator, index ascending, every add

@@ -34,7 +34,6 @@
 
 namespace apus {
 
-__device__ int g_tc_status = 0;
 
 namespace {
 
@@ -275,7 +274,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     }
     if (fail) {
         *s_abort = 1;
-        atomicCAS(&g_tc_status, 0, fail);
+        atomicCAS(a.status, 0, fail);
     }
     if (S > 1) {
         // the chunk that arrives last at this (tile, work item) adds the chunks in order and finishes the rows
@@ -397,6 +396,7 @@ int gemm_tc(const TcArgs &a0, cudaStream_t st) {
             a.ksplit = S; a.part = (float *)ws; a.counters = cnt;
         }
     }
+    if (!(a.status = wait_word())) return 1;
     if (a.rows64 && a.pair) return launch_tc<true, 2, 64>(a, st);
     if (a.rows64) return launch_tc<false, 4, 64>(a, st);
     static const int pns = getenv("APUS_TC_PAIR_NS") ? atoi(getenv("APUS_TC_PAIR_NS")) : 3;
@@ -408,21 +408,6 @@ int gemm_tc(const TcArgs &a0, cudaStream_t st) {
     if (ns == 2) return launch_tc<false, 2>(a, st);
     if (ns == 3) return launch_tc<false, 3>(a, st);
     return launch_tc<false, 5>(a, st);
-}
-
-// Status word of the bounded waits (0 = no failure since the last reset).
-int gemm_tc_status(int reset) {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_tc_status, sizeof(int)) != cudaSuccess) return -1;
-    if (reset && v) {
-        int z = 0;
-        cudaMemcpyToSymbol(g_tc_status, &z, sizeof(int));
-    }
-    const int v8 = gemm_tc8_status(reset);          // the FP8 kernel keeps its own word (codes 11..15)
-    const int vb = gemm_tcbf_status(reset);         // and the BF16 kernel (codes 21..23)
-    const int va = attn_status(reset);              // and P.V of the sparse attention (31)
-    const int vl = linear_status(reset);            // and the chain linears (41, 42)
-    return v ? v : (v8 ? v8 : vb ? vb : va ? va : vl);
 }
 
 }  // namespace apus

@@ -29,7 +29,6 @@
 
 namespace apus {
 
-__device__ int g_tc8_status = 0;         // first failure code (11..16) recorded by any CTA
 
 namespace {
 
@@ -223,7 +222,7 @@ gemm_tc8_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     }
     if (fail) {
         *s_abort = 1;
-        atomicCAS(&g_tc8_status, 0, fail);
+        atomicCAS(a.status, 0, fail);
     }
     if (S > 1) {
         // the chunk that arrives last at this output tile adds every block's term in block order and finishes the rows
@@ -431,7 +430,7 @@ gemm_tc8_wide_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     }
     if (fail) {
         *s_abort = 1;
-        atomicCAS(&g_tc8_status, 0, fail);
+        atomicCAS(a.status, 0, fail);
         for (int i = 0; i < 2000; i++) __nanosleep(1000);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -475,12 +474,13 @@ int tc8_make_weight_map(void *out_map, const void *codes, long long rows, int K)
 }
 
 // a.map_x must be a map with 128-row boxes (tc8_make_act_map_wide)
-int gemm_tc8_wide(const Tc8Args &a, cudaStream_t st) {
+int gemm_tc8_wide(const Tc8Args &a0, cudaStream_t st) {
+    Tc8Args a = a0;
     APUS_REQUIRE(a.K % 128 == 0 && a.K <= 128 * 64 && a.O % 128 == 0 && !a.pair,
                  "gemm_tc8_wide: unsupported shape O=%d K=%d", a.O, a.K);
     if (a.M <= 0) return 0;
     const size_t smem = (size_t)T8W_NS * T8W_STAGE + T8W_NACC * T8W_N * 4 + 1024 + 256;
-    if (ensure_dyn_smem((const void *)gemm_tc8_wide_kernel, smem)) return 1;
+    if (!(a.status = wait_word()) || ensure_dyn_smem((const void *)gemm_tc8_wide_kernel, smem)) return 1;
     int dev = 0, sms = 0;
     APUS_CUDA_OK(cudaGetDevice(&dev));
     APUS_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -523,20 +523,11 @@ int gemm_tc8(const Tc8Args &a0, cudaStream_t st) {
             ctas *= S;
         }
     }
+    if (!(a.status = wait_word())) return 1;
     // few CTAs: one CTA per SM with a deep ring, so that each CTA keeps ~200 KB of weight
     // tiles in flight; many CTAs: two per SM with a short ring
     if (a.pair) return ctas <= 148 ? launch_tc8<true, 5>(a, st) : launch_tc8<true, 3>(a, st);
     return ctas <= 148 ? launch_tc8<false, 10>(a, st) : launch_tc8<false, 4>(a, st);
-}
-
-int gemm_tc8_status(int reset) {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_tc8_status, sizeof(int)) != cudaSuccess) return -1;
-    if (reset && v) {
-        int z = 0;
-        cudaMemcpyToSymbol(g_tc8_status, &z, sizeof(int));
-    }
-    return v;
 }
 
 }  // namespace apus

@@ -25,7 +25,6 @@
 
 namespace apus {
 
-__device__ int g_tcbf_status = 0;        // first failure code (21..24) recorded by any CTA
 
 namespace {
 
@@ -151,7 +150,7 @@ gemm_tcbf_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     }
     if (fail) {
         *s_abort = 1;
-        atomicCAS(&g_tcbf_status, 0, fail);
+        atomicCAS(a.status, 0, fail);
     }
     if (S > 1) {
         // the chunk that arrives last at this output tile adds the chunks in order
@@ -327,7 +326,7 @@ gemm_tcbf_wide_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
     }
     if (fail) {
         *s_abort = 1;
-        atomicCAS(&g_tcbf_status, 0, fail);
+        atomicCAS(a.status, 0, fail);
         for (int i = 0; i < 2000; i++) __nanosleep(1000);   // copies already issued to this CTA's shared memory land
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -397,9 +396,11 @@ int tcbf_ksplit(int O, int K, int batch, int M) {
     return s < 1 ? 1 : s;
 }
 
-int gemm_tcbf(const TcbfArgs &a, cudaStream_t st) {
+int gemm_tcbf(const TcbfArgs &a0, cudaStream_t st) {
+    TcbfArgs a = a0;
     APUS_REQUIRE(a.K % TB_KT == 0 && a.O % 128 == 0 && a.batch >= 1, "gemm_tcbf: unsupported shape O=%d K=%d", a.O, a.K);
     if (a.M <= 0) return 0;
+    if (!(a.status = wait_word())) return 1;
     const int S = a.ksplit < 1 ? 1 : a.ksplit;
     APUS_REQUIRE(S == 1 || (a.part && a.counters), "gemm_tcbf: a K split needs the scratch buffers");
     APUS_REQUIRE(!a.q_out || (S > 1 && a.qs_out && a.out_ld % 128 == 0), "gemm_tcbf: codes are written by the K-split finish only");
@@ -430,16 +431,6 @@ int gemm_tcbf(const TcbfArgs &a, cudaStream_t st) {
     }
     APUS_LAUNCHED();
     return 0;
-}
-
-int gemm_tcbf_status(int reset) {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_tcbf_status, sizeof(int)) != cudaSuccess) return -1;
-    if (reset && v) {
-        int z = 0;
-        cudaMemcpyToSymbol(g_tcbf_status, &z, sizeof(int));
-    }
-    return v;
 }
 
 }  // namespace apus

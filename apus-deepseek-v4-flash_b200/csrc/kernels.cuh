@@ -85,9 +85,9 @@ struct TcArgs {
     int ksplit;                          // set by gemm_tc: K chunks (grid.z); > 1 uses part + counters
     float *part;                         // [(pair ? 2 : 1) * ksplit, total_rows, O] chunk sums
     int *counters;                       // zeroed, one per (output tile, work item); left zeroed
+    int *status;                         // set by gemm_tc: wait_word()
 };
 int gemm_tc(const TcArgs &a, cudaStream_t st);
-int gemm_tc_status(int reset);
 int tc_make_weight_map(void *out_map, const void *codes, long long rows, int K);
 int tc_make_act_map(void *out_map, const void *codes, long long rows, int K, int box_rows = 32);
 
@@ -102,11 +102,11 @@ struct Tc8Args {
     int ksplit;                          // set by gemm_tc8: K chunks (grid.z); > 1 uses part + counters
     float *part;                         // [(pair ? 2 : 1) * K/128, M, O] per-block terms
     int *counters;                       // zeroed, one per (output tile, row group); left zeroed
+    int *status;                         // set by gemm_tc8 / gemm_tc8_wide: wait_word()
 };
 int gemm_tc8(const Tc8Args &a, cudaStream_t st);
 int gemm_tc8_wide(const Tc8Args &a, cudaStream_t st);      // 128 activation rows per CTA; map_x from tc8_make_act_map_wide
 int tc8_make_act_map_wide(void *out_map, const void *codes, long long rows, int K);
-int gemm_tc8_status(int reset);
 int tc8_make_weight_map(void *out_map, const void *codes, long long rows, int K);
 
 // ---- tcgen05 BF16 GEMM on row-major BF16 weights (gemm_tcbf.cu) ---------------------------
@@ -123,9 +123,9 @@ struct TcbfArgs {
     int *counters;                       // zeroed, one per (output tile, row group); left zeroed
     uint8_t *q_out;                      // ksplit > 1, out_ld % 128 == 0: also the E4M3 activation codes [M, out_ld] ...
     float *qs_out;                       // ... and per-128 scales [M, out_ld / 128] of the finished rows (act_quant's)
+    int *status;                         // set by gemm_tcbf: wait_word()
 };
 int gemm_tcbf(const TcbfArgs &a, cudaStream_t st);
-int gemm_tcbf_status(int reset);
 int tcbf_ksplit(int O, int K, int batch, int M);
 int tcbf_make_weight_map(void *out_map, const void *w_bf16, long long rows, int K);
 bool tcbf_wide(int M, int S);             // M rows with S K chunks go to the 128-row tiles (no scratch, no codes)
@@ -153,7 +153,6 @@ struct LinCodes {
     float *s;
     int written;
 };
-int linear_status(int reset);             // status word of the bounded waits in the f32 linears (0 = none expired)
 int f32_linear_batched(const void *w, long long w_stride, const float *x, long long x_stride, int x_ld,
                        float *out, long long out_stride, int out_ld, int batch, int M, int K, int O,
                        int flags, cudaStream_t st, LinCodes *codes = nullptr);
@@ -202,7 +201,6 @@ int sparse_attn(const float *q, const float *sink, int h, int d,
                 bool ids_ready = false,              // sparse_attn_compact has run on this scratch with these index rows
                 const struct SaRope *rope = nullptr);   // rotate the output rows back before they are written
 size_t sparse_attn_scratch(int h, int idxw, int s);
-int attn_status(int reset);               // status word of the bounded waits in P.V (0 = none expired)
 // The first launch of sparse_attn (negative ids dropped, order kept) on its own: a caller that has the
 // index rows before the queries (a side chain) runs it there, into the scratch it then hands to sparse_attn.
 int sparse_attn_compact(const int32_t *idxs, int h, int idxw, int s, void *scratch, size_t scratch_cap, cudaStream_t st);

@@ -384,7 +384,6 @@ f32_linear_seq_kernel(const void *__restrict__ wv, const float *__restrict__ x, 
 // One chain per lane walks at 4.14 cycles per k.  (Bulk copies, one per row, were
 // slower than the kernel above: some 33 cycles each whatever their size.)  B200, K = 4096: one token
 // 24.4 -> 19.3 us, two to eight tokens 34 -> 19 us, 32 tokens x 256 rows (the gate) 26.6 -> 17.5 us.
-__device__ int g_linear_status = 0;       // 41 / 42: a wait of the producer / of a chain warp expired
 template <int MTT, int CW, int NST>
 struct ChainCfg {
     static constexpr int TOK = MTT * CW, XBOX = TOK * 128 < 1024 ? 1024 : TOK * 128;        // bytes of a 32-wide box of x
@@ -395,7 +394,7 @@ template <int MTT, int CW, int NST>
 __global__ void __launch_bounds__(32 * (CW + 1))
 f32_chain_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
                  const __grid_constant__ CUtensorMap tm_x, float *__restrict__ out, int M, int K, int O, int flags,
-                 long long out_stride, int out_ld) {
+                 long long out_stride, int out_ld, int *__restrict__ status) {
     APUS_PDL_WAIT();
     APUS_PDL_GO();
     using Cf = ChainCfg<MTT, CW, NST>;
@@ -492,19 +491,9 @@ f32_chain_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constan
     }
     if (fail) {
         s_abort = 1;
-        atomicCAS(&g_linear_status, 0, fail);
+        atomicCAS(status, 0, fail);                            // 41 / 42: a wait of the producer / of a chain warp
         for (int i = 0; i < 2000; i++) __nanosleep(1000);      // copies already issued to this CTA's shared memory land
     }
-}
-
-int linear_status(int reset) {
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_linear_status, sizeof(int)) != cudaSuccess) return -1;
-    if (reset && v) {
-        int z = 0;
-        cudaMemcpyToSymbol(g_linear_status, &z, sizeof(int));
-    }
-    return v;
 }
 
 // Tensor map over f32 rows [rows, K], `ld` floats apart, boxes of 32 x box_rows
@@ -524,14 +513,15 @@ static int chain_launch(const float *w, long long ws, const float *x, int x_ld, 
                         int batch, int M, int K, int O, int flags, cudaStream_t st) {
     using Cf = ChainCfg<MTT, CW, NST>;
     auto kern = f32_chain_kernel<MTT, CW, NST>;
-    if (ensure_dyn_smem((const void *)kern, Cf::SMEM + 16)) return 1;
+    int *status = wait_word();
+    if (!status || ensure_dyn_smem((const void *)kern, Cf::SMEM + 16)) return 1;
     alignas(64) unsigned char m0[128], m1[128], mx[128];
     if (make_f32_map(m0, w, O, K, K, 32) || make_f32_map(m1, w + (batch > 1 ? ws : 0), O, K, K, 32) ||
         make_f32_map(mx, x, M, K, x_ld, Cf::TOK))
         return 1;
     const dim3 grid((unsigned)ceil_div(O, 32), (unsigned)ceil_div(M, Cf::TOK), (unsigned)batch);
     launch_k(kern, grid, 32 * (CW + 1), Cf::SMEM, st, *reinterpret_cast<const CUtensorMap *>(m0),
-             *reinterpret_cast<const CUtensorMap *>(m1), *reinterpret_cast<const CUtensorMap *>(mx), out, M, K, O, flags, os, out_ld);
+             *reinterpret_cast<const CUtensorMap *>(m1), *reinterpret_cast<const CUtensorMap *>(mx), out, M, K, O, flags, os, out_ld, status);
     return 0;
 }
 

@@ -633,7 +633,7 @@ int apus_cuda_f32_linear(const float *w, const float *x, float *out, int M, int 
     if (f32_linear(dw, (float *)dx, (float *)dout, M, K, O, flags, c.stream)) return 1;
     APUS_CUDA_OK(cudaMemcpyAsync(out, dout, (size_t)M * O * 4, cudaMemcpyDeviceToHost, c.stream));
     APUS_CUDA_OK(cudaStreamSynchronize(c.stream));
-    return 0;
+    return wait_check("f32_linear");
 }
 
 int apus_cuda_head_gemv_bf16(const void *w_bf16, const float *x, float *out, int64_t O,
@@ -833,7 +833,7 @@ int apus_cuda_expert(const void *w1, const void *w2, const void *w3, int kind, f
     if (expert_dev(d1, d2, d3, limit, (float *)dx, rows, (float *)dout, ws, c.stream)) return 1;
     APUS_CUDA_OK(cudaMemcpyAsync(out, dout, (size_t)rows * dim * 4, cudaMemcpyDeviceToHost, c.stream));
     APUS_CUDA_OK(cudaStreamSynchronize(c.stream));
-    return 0;
+    return wait_check("expert");
 }
 
 int apus_cuda_topk_stable(const float *row, int n, int k, int32_t *idx, int rows) {
@@ -871,7 +871,7 @@ int apus_cuda_sparse_attn(const float *q, const float *sink, int h, int d, const
         return 1;
     APUS_CUDA_OK(cudaMemcpyAsync(o, dout, qb, cudaMemcpyDeviceToHost, c.stream));
     APUS_CUDA_OK(cudaStreamSynchronize(c.stream));
-    return 0;
+    return wait_check("sparse_attn");
 }
 
 // ---- mHC host-pointer entry points ------------------------------------------------------------

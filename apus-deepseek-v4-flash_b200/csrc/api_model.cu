@@ -1638,7 +1638,7 @@ int apus_cuda_dspark_feed(ApusCudaDspark *ds, const float *mh, int64_t pos0, int
     APUS_CUDA_OK(cudaMemcpyAsync(ds->mh.p, mh, (size_t)n * mhd * 4, cudaMemcpyHostToDevice, st));
     if (ds_project(ds, ds->mh.as<float>(), n, st) || ds_ring_rows(ds, n, pos0, st)) return 1;
     APUS_CUDA_OK(cudaStreamSynchronize(st));
-    return 0;
+    return wait_check("dspark_feed");
 }
 
 // c/dspark.h:611 apus_dspark_draft_round, greedy drafts: mh_row [n_targets * dim] (host) = main hidden of position

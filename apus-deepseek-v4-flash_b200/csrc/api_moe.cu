@@ -601,7 +601,7 @@ int apus_cuda_router_score(const ApusMoeW *w, const float *x, int s, float *sp, 
     APUS_CUDA_OK(cudaMemcpyAsync(sp, dsp, se, cudaMemcpyDeviceToHost, c.stream));
     if (biased) APUS_CUDA_OK(cudaMemcpyAsync(biased, db, se, cudaMemcpyDeviceToHost, c.stream));
     APUS_CUDA_OK(cudaStreamSynchronize(c.stream));
-    return 0;
+    return wait_check("router_score");
 }
 
 int apus_cuda_moe_forward(const ApusMoeW *w, const float *x, const int64_t *ids, int s, float *out,
@@ -644,10 +644,7 @@ int apus_cuda_moe_forward(const ApusMoeW *w, const float *x, const int64_t *ids,
         if (interm->moe_shared) APUS_CUDA_OK(cudaMemcpyAsync(interm->moe_shared, m->b_shared.p, sd, cudaMemcpyDeviceToHost, c.stream));
     }
     APUS_CUDA_OK(cudaStreamSynchronize(c.stream));
-    if (m->use_tc) {
-        if (wait_check("moe_forward")) return 1;
-    }
-    return 0;
+    return wait_check("moe_forward");
 }
 
 int apus_cuda_kernel_status(int reset) { return wait_status(reset); }

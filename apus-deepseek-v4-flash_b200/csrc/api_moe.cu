@@ -103,6 +103,17 @@ static int pick_chunk(int n_rout, int n_local) {
     return 32;
 }
 
+// Rows per work item of the expert GEMMs.  A weight tile is read once per item, so experts with more than 32 rows want
+// items of 64; with fewer, the wider MMA and the shallower ring cost and bring nothing.  What counts is the routings to
+// be expected per local expert: of the slots of a padded exchange, sized for every routing of every rank, one in
+// n_experts / n_local is filled.  B200, gate/up and down together with items of 32 / 64: 24 rows per expert 874 / 990 us,
+// 28 rows 977 / 1,035, 33 rows 1,172 / 1,092, 48 rows 1,557 / 1,380; a shard of 32 experts with 3 rows each (18 tokens on
+// each of 8 ranks) 101 / 120, 24 rows 156 / 160, 30 rows 189 / 172.  The sums are the same.
+int apus::tc_item_rows(long long slots, int n_local, int n_experts, bool padded) {
+    const long long live = padded ? slots * n_local / n_experts : slots;
+    return live > 29LL * n_local ? 64 : 32;
+}
+
 // Routed experts on the tcgen05 path: group first, quantise the token rows
 // straight into sorted order, then two block-scaled tensor-core GEMMs.
 // qrows != NULL: the token rows arrive quantised (EP exchange: dim codes + dim/128 scales per row,
@@ -113,11 +124,8 @@ static int experts_run_tc(ApusCudaMoe *m, const float *xrows, const int32_t *rou
                           const uint8_t *qrows = nullptr) {
     const int dim = m->dim, inter = m->inter;
     const int n_local = m->e_hi - m->e_lo;
-    // Rows per work item.  A weight tile is read once per item, so experts with more than 32 rows want items of 64;
-    // with fewer, the wider MMA and the shallower ring cost and bring nothing.  B200, 2,048 tokens (48 rows
-    // per expert): gate/up 1,062 -> 925 us, down 465 -> 405 us.  The sums are the same.
-    const bool rows64 = n_rout > 26LL * n_local;
-    const int chunk = rows64 ? 64 : 32;
+    const int chunk = tc_item_rows(n_rout, n_local, m->E, qrows != nullptr);
+    const bool rows64 = chunk == 64;
     const int max_groups = n_rout < n_local + n_rout / chunk + 1 ? n_rout : n_local + n_rout / chunk + 1;
     int *ng = m->b_ng.as<int>();
     if (moe_group(rout_eid, rout_row, qrows ? 1 : m->topk, n_rout, m->sl, chunk, m->b_spos.as<int>(), m->b_srow.as<int>(),

@@ -88,6 +88,7 @@ struct TcArgs {
     int *status;                         // set by gemm_tc: wait_word()
 };
 int gemm_tc(const TcArgs &a, cudaStream_t st);
+int tc_item_rows(long long slots, int n_local, int n_experts, bool padded);     // rows per work item: 32 or 64 (api_moe.cu)
 int tc_make_weight_map(void *out_map, const void *codes, long long rows, int K);
 int tc_make_act_map(void *out_map, const void *codes, long long rows, int K, int box_rows = 32);
 

@@ -154,6 +154,7 @@ struct LinCodes {
     float *s;
     int written;
 };
+bool seq64_pays(long long ctas32, long long ctas64);     // dispatch of the f32 linears of many tokens (linear.cu)
 int f32_linear_batched(const void *w, long long w_stride, const float *x, long long x_stride, int x_ld,
                        float *out, long long out_stride, int out_ld, int batch, int M, int K, int O,
                        int flags, cudaStream_t st, LinCodes *codes = nullptr);

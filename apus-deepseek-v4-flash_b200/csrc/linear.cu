@@ -525,6 +525,12 @@ static int chain_launch(const float *w, long long ws, const float *x, int x_ld, 
     return 0;
 }
 
+// f32 weights, 32 tokens per CTA: a CTA of 64 output rows (two per lane) takes 11/7 of the time of one of 32 rows, and
+// an SM works through one after another, so the taller tile pays unless it saves too few waves of 148.  B200, K = 4096,
+// tiles of 32 / 64 rows: 32 tokens x 4,736 rows (148 / 74 CTAs) 78 / 121 us, x 9,472 (296 / 148) 155 / 123, x 9,504
+// (297 / 149) 223 / 235; 2,048 tokens x 1,024 rows 1,060 / 850.
+bool seq64_pays(long long ctas32, long long ctas64) { return (ctas64 + 147) / 148 * 11 < (ctas32 + 147) / 148 * 7; }
+
 template <bool WBF16, int R, int MTT, int MG, int NST>
 static cudaError_t seq_launch(cudaStream_t st, int batch, const void *w, const float *x, float *out, int M, int K,
                               int O, int flags, long long ws, long long xs, int x_ld, long long os, int out_ld) {
@@ -572,7 +578,9 @@ static int launch_linear_seq(const void *w, long long ws, const float *x, long l
     else if (M > 8 && ctas32 < 32) SEQ_LAUNCH(1, 1, 4, 6);      // 4 tokens per CTA, one per warp
     else if (M <= 8 || ctas32 < 64) SEQ_LAUNCH(1, 2, 4, 6);     // 8 tokens per CTA, two per warp
     else if (M <= 16 || ctas32 < 148) SEQ_LAUNCH(1, 2, 8, 3);   // 16 tokens per CTA
-    else SEQ_LAUNCH(2, 4, 8, 3);                                // 32 tokens x 64 rows per CTA
+    else if (WBF16 || seq64_pays(ctas32, (long long)ceil_div(O, 64) * batch * ceil_div(M, 32)))
+        SEQ_LAUNCH(2, 4, 8, 3);                                 // 32 tokens x 64 rows per CTA
+    else if constexpr (!WBF16) SEQ_LAUNCH(1, 4, 8, 3);          // 32 tokens x 32 rows
 #undef SEQ_LAUNCH
     return 0;
 }

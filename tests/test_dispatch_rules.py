@@ -25,3 +25,11 @@ def test_item_rows_follow_the_routings_to_be_expected():
     for tokens, want in ((512, 32), (1200, 32), (1400, 64), (2048, 64)):
         assert rows(tokens * topk, E, E, False) == want
     assert rows(0, 0, E, True) == 32
+
+
+def test_taller_tiles_of_the_f32_linears_only_where_they_save_waves():
+    pays = rule("_ZN4apus10seq64_paysExx", C.c_bool, C.c_longlong, C.c_longlong)
+    up = lambda a, b: -(-a // b)   # noqa: E731
+    for tokens, rows, want in ((32, 4736, False), (32, 4768, True), (32, 9472, True), (32, 9504, False), (320, 1024, False), (512, 1024, True),
+                               (2048, 1024, True)):
+        assert pays(up(rows, 32) * up(tokens, 32), up(rows, 64) * up(tokens, 32)) == want, (tokens, rows)

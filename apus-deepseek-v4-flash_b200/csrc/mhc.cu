@@ -36,6 +36,7 @@ __device__ __forceinline__ float block_sum(float v, float *red) {
 
 // grid (nmix + 1, rows): blockIdx.x < nmix -> raw[row, j] = fn_j . x ;
 // blockIdx.x == nmix -> raw[row, nmix] = sum x^2.
+template <int U>
 __global__ void __launch_bounds__(256)
 mhc_mix_kernel(const float *__restrict__ x4, const float *__restrict__ fn, int nx, int nmix,
                float *__restrict__ raw) {
@@ -47,11 +48,14 @@ mhc_mix_kernel(const float *__restrict__ x4, const float *__restrict__ fn, int n
     float acc = 0.f;
     if (j < nmix) {
         const float *f = fn + (size_t)j * nx;
-        // the loads of eight steps are issued before the sums that use them: the kernel is a chain of L2 latencies
-        for (int i0 = threadIdx.x * 4; i0 < nx; i0 += blockDim.x * 32) {
-            float4 a[8], b[8];
+        // U = 8: the loads of eight steps are issued before the sums that use them.  With few CTAs the kernel is a chain
+        // of L2 latencies; with more than two per SM the others hide them and the registers cost.  B200, 24 x 16384: one
+        // row 6.1 -> 4.5 us, 10 rows 6.4 -> 5.1; 12 rows 6.4 with one step at a time, 6.8 with eight, 32 rows 7.0 / 10.0,
+        // 128 rows 19.6 / 29.5; 24 x 4096, one row 2.8 / 2.2, 24 x 1024 1.9 / 2.1.
+        for (int i0 = threadIdx.x * 4; i0 < nx; i0 += blockDim.x * 4 * U) {
+            float4 a[U], b[U];
 #pragma unroll
-            for (int u = 0; u < 8; u++) {
+            for (int u = 0; u < U; u++) {
                 const int i = i0 + u * blockDim.x * 4;
                 if (i < nx) {
                     a[u] = __ldg(reinterpret_cast<const float4 *>(f + i));
@@ -59,7 +63,7 @@ mhc_mix_kernel(const float *__restrict__ x4, const float *__restrict__ fn, int n
                 }
             }
 #pragma unroll
-            for (int u = 0; u < 8; u++)
+            for (int u = 0; u < U; u++)
                 if (i0 + u * blockDim.x * 4 < nx) {
                     acc = fmaf(a[u].x, b[u].x, acc); acc = fmaf(a[u].y, b[u].y, acc);
                     acc = fmaf(a[u].z, b[u].z, acc); acc = fmaf(a[u].w, b[u].w, acc);
@@ -682,14 +686,20 @@ static float *ensure_raw(size_t floats, float *callers) {
 // raw[row, 0..nmix] for `rows` tokens in the sum order now in force.
 static int launch_mix(const float *x4, const float *fn, int nx, int nmix, float *raw, int rows,
                       cudaStream_t st) {
-    if (sum_tree(APUS_CUDA_TREE_MHC_MAPS) && rows >= 256) {      // a CTA per 8 rows still fills the SMs
+    const long long rows_ctas = (long long)ceil_div(nmix + 1, 5) * ceil_div(rows, 8);
+    // (one by one / in eights: n = 2, d = 1024 300 rows, 76 CTAs, 5.4 / 5.7 us, 512 rows, 128 CTAs, 7.6 / 5.9; the head's
+    // five dots of 16384 at 256 rows, 32 CTAs, 12.1 / 22.4, 768 rows, 96 CTAs, 25.6 / 25.1)
+    if (sum_tree(APUS_CUDA_TREE_MHC_MAPS) && rows >= 256 && rows_ctas >= 96) {      // a CTA per 8 rows still fills the SMs
         launch_k(mhc_mix_rows_kernel<8, 5>, dim3((unsigned)ceil_div(nmix + 1, 5), (unsigned)ceil_div(rows, 8)), 256, 0, st, x4, fn, nx,
                  nmix, rows, raw);
         APUS_LAUNCHED();
         return 0;
     }
     if (sum_tree(APUS_CUDA_TREE_MHC_MAPS)) {
-        launch_k(mhc_mix_kernel, dim3(nmix + 1, rows), 256, 0, st, x4, fn, nx, nmix, raw);
+        if (nx >= 4096 && (long long)(nmix + 1) * rows <= 2 * 148)
+            launch_k(mhc_mix_kernel<8>, dim3(nmix + 1, rows), 256, 0, st, x4, fn, nx, nmix, raw);
+        else
+            launch_k(mhc_mix_kernel<1>, dim3(nmix + 1, rows), 256, 0, st, x4, fn, nx, nmix, raw);
         APUS_LAUNCHED();
         return 0;
     }

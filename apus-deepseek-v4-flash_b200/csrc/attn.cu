@@ -1152,14 +1152,19 @@ static int attn_tiled(const float *q, const float *sink, int h, int d, const int
                       float scale, const void *kv_a, int64_t na, const void *kv_b, float *sc, float *den, int *bad, float *o,
                       cudaStream_t st, size_t sa, size_t sb, int seq_mod, const SaRope &rope) {
 #define SA_ARGS q, h, d, ids, ns, idxw, s, scale, kv_a, na, kv_b, sc, bad, st, sa, sb, seq_mod
-    // The larger a lane's tile, the fewer shared loads per multiply-add; the smaller, the more warps share the work
-    // of a small step.  Lines drawn where the measured times cross (64 heads, d = 512, BF16 rows; us with 16 heads x
-    // 32 candidates of 4 x 1 per lane / 16 x 32 of 4 x 2 / 64 x 64 of 4 x 4): 1 row of 640 candidates 11.6 / 15.0 /
-    // 25.1, 2 rows 16.4 / 15.6 / 25.4, 4 rows 20.8 / 19.2 / 25.6, 7 rows of 909 38 / 26.7 / 26.0, 32 rows of 640
-    // 107 / 76 / 62 (96 before).
-    const long long c64 = (long long)ceil_div(idxw, 64) * ceil_div(h, 64) * s;
-    if (c64 < 15) { if (scores_launch<BF16, 4, 1, 1, 4>(SA_ARGS)) return 1; }
-    else if (c64 < 80) { if (scores_launch<BF16, 4, 2, 1, 2>(SA_ARGS)) return 1; }
+    // The larger a lane's tile, the fewer shared loads per multiply-add; the smaller, the more warps share the work of a
+    // small step.  Three sizes of work, counted in 16-head tiles so that a head count below 64 is not taken for more than
+    // it is (us, BF16 rows, d = 512, with 16 heads x 32 candidates of 4 x 1 per lane / 16 x 32 of 4 x 2 / the large tile):
+    // the smallest tile while its CTAs have an SM each (64 heads: 1 row of 909 11.8 / 15.2 / 25, 2 rows of 640, 160 CTAs,
+    // 16.3 / 15.4 / 25; 32 rows of 16 10.7 / 14.9 / 19), the large one when it has 80 tiles of 64 x 64 (8 rows of 640 32 /
+    // 24.4 / 25.5, 32 rows 107 / 76 / 61).  The large one is as tall as the heads: 4 x 4 per lane, 64 heads x 64
+    // candidates, 32 x 64 or 16 x 128 (8 heads: 256 rows of 640 129 / 96 as 16 x 128, 224 as 64 x 64; 32 heads: 253 / 178
+    // as 32 x 64, 320), unless the rows are shorter than a tile is wide (8 heads, 1,024 rows of 16: 29 / 53).
+    const long long ctas0 = (long long)ceil_div(idxw, 32) * ceil_div(h, 16) * s, c16 = (long long)ceil_div(idxw, 64) * ceil_div(h, 16) * s;
+    if (ctas0 <= 148) { if (scores_launch<BF16, 4, 1, 1, 4>(SA_ARGS)) return 1; }
+    else if (c16 < 320 || (h <= 32 && idxw <= 32)) { if (scores_launch<BF16, 4, 2, 1, 2>(SA_ARGS)) return 1; }
+    else if (h <= 16) { if (scores_launch<BF16, 4, 4, 1, 4>(SA_ARGS)) return 1; }
+    else if (h <= 32) { if (scores_launch<BF16, 4, 4, 2, 2>(SA_ARGS)) return 1; }
     else if (scores_launch<BF16, 4, 4, 4, 2>(SA_ARGS)) return 1;
 #undef SA_ARGS
     // a warp per row once that is a warp and more for every scheduler; with fewer rows the exponentials want a CTA per

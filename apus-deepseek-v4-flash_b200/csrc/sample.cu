@@ -34,7 +34,7 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-constexpr int SMP_THREADS = 1024, SMP_CL = 8;
+constexpr int SMP_THREADS = 1024;
 constexpr int SMP_BATCH = 1 << 17;                        // elements of a slice between flushes of the 32-bit counters
 constexpr double SMP_ONE = 1152921504606846976.0;        // 2^60
 
@@ -63,8 +63,8 @@ struct Sel {                 // answer of first_exceed
 };
 
 // First token, in (p desc, index asc) order, whose inclusive prefix mass exceeds M: every thread of the
-// cluster gets the same found / key / above / k.  p: this slice's np probabilities.  `buf` is the histogram
-// buffer to start with; the caller alternates.
+// cluster (CL CTAs) gets the same found / key / above / k.  p: this slice's np probabilities.  row_mass (may be null): the row's mass.
+template <int CL>
 __device__ __forceinline__ Sel first_exceed(cg::cluster_group &cluster, SmpShared &S, const float *p, int np,
                                             unsigned long long M, unsigned long long *row_mass) {
     const int tid = threadIdx.x, lane = tid & 31;
@@ -106,7 +106,7 @@ __device__ __forceinline__ Sel first_exceed(cg::cluster_group &cluster, SmpShare
         if (tid < 256) {
             unsigned long long t = 0;
 #pragma unroll
-            for (int q = 0; q < SMP_CL; q++) t += *cluster.map_shared_rank(&S.mass[buf][tid], q);
+            for (int q = 0; q < CL; q++) t += *cluster.map_shared_rank(&S.mass[buf][tid], q);
             S.tot[tid] = t;
         }
         __syncthreads();
@@ -149,7 +149,7 @@ __device__ __forceinline__ Sel first_exceed(cg::cluster_group &cluster, SmpShare
             const unsigned long long pm = mass_of(__uint_as_float(prefix));
             unsigned long long ties = 0;
             const int rank = (int)cluster.block_rank();
-            for (int q = 0; q < SMP_CL; q++) {
+            for (int q = 0; q < CL; q++) {
                 const unsigned long long n = *cluster.map_shared_rank(&S.mass[buf][b], q) / pm;
                 if (q == rank) { r.before = ties; r.here = n; }
                 ties += n;
@@ -165,7 +165,8 @@ __device__ __forceinline__ Sel first_exceed(cg::cluster_group &cluster, SmpShare
 }
 
 // u == NULL: the row's uniform comes from its splitmix64 state (advanced here).
-__global__ void __cluster_dims__(SMP_CL, 1, 1) __launch_bounds__(SMP_THREADS)
+template <int CL>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(SMP_THREADS)
 sample_rows_kernel(const float *__restrict__ logits, int n, float temp, float top_p,
                    const double *__restrict__ u_in, unsigned long long *__restrict__ rng,
                    float *probs, int in_smem, int32_t *__restrict__ out) {
@@ -174,8 +175,8 @@ sample_rows_kernel(const float *__restrict__ logits, int n, float temp, float to
     extern __shared__ float s_slice[];
     __shared__ SmpShared S;
     cg::cluster_group cluster = cg::this_cluster();
-    const int row = blockIdx.x / SMP_CL, rank = (int)cluster.block_rank(), tid = threadIdx.x, lane = tid & 31;
-    const int per = (n + SMP_CL - 1) / SMP_CL, i0 = min(n, rank * per), np = min(n, i0 + per) - i0;
+    const int row = blockIdx.x / CL, rank = (int)cluster.block_rank(), tid = threadIdx.x, lane = tid & 31;
+    const int per = (n + CL - 1) / CL, i0 = min(n, rank * per), np = min(n, i0 + per) - i0;
     const float *l = logits + (size_t)row * n + i0;
     float *p = in_smem ? s_slice : probs + (size_t)row * n + i0;
     // max
@@ -194,7 +195,7 @@ sample_rows_kernel(const float *__restrict__ logits, int n, float temp, float to
     }
     cluster.sync();
 #pragma unroll
-    for (int q = 0; q < SMP_CL; q++) { const float v = *cluster.map_shared_rank(&S.mxpart, q); mx = q ? fmaxf(mx, v) : v; }
+    for (int q = 0; q < CL; q++) { const float v = *cluster.map_shared_rank(&S.mxpart, q); mx = q ? fmaxf(mx, v) : v; }
     // softmax: f32 exponent argument, double sum (a tree here), one rounding back to f32
     double part = 0.0;
     for (int i = tid; i < np; i += SMP_THREADS) {
@@ -215,7 +216,7 @@ sample_rows_kernel(const float *__restrict__ logits, int n, float temp, float to
     cluster.sync();
     double sum = 0.0;
 #pragma unroll
-    for (int q = 0; q < SMP_CL; q++) sum += *cluster.map_shared_rank(&S.part, q);
+    for (int q = 0; q < CL; q++) sum += *cluster.map_shared_rank(&S.part, q);
     for (int i = tid; i < np; i += SMP_THREADS) p[i] = (float)((double)p[i] / sum);
     // the row's uniform
     double u;
@@ -233,11 +234,11 @@ sample_rows_kernel(const float *__restrict__ logits, int n, float temp, float to
     // (top_p >= 1.5 can never be exceeded by probabilities: then this call only adds up the row's mass)
     const double tp = (double)top_p;
     unsigned long long total = 0;
-    const Sel cut = first_exceed(cluster, S, p, np, tp >= 1.5 ? ~0ull : tp <= 0.0 ? 0ull : (unsigned long long)(tp * SMP_ONE), &total);
+    const Sel cut = first_exceed<CL>(cluster, S, p, np, tp >= 1.5 ? ~0ull : tp <= 0.0 ? 0ull : (unsigned long long)(tp * SMP_ONE), &total);
     const unsigned long long kept = cut.found ? cut.above + cut.k * mass_of(__uint_as_float(cut.key)) : total;
     // draw inside the kept mass
     const unsigned long long Mu = (unsigned long long)(u * (double)kept);
-    const Sel d = first_exceed(cluster, S, p, np, Mu < kept ? Mu : kept - 1, nullptr);
+    const Sel d = first_exceed<CL>(cluster, S, p, np, Mu < kept ? Mu : kept - 1, nullptr);
     if (!d.found) {                                          // no mass at all (logits without a finite maximum)
         if (rank == 0 && tid == 0) out[row] = 0;
         return;
@@ -269,19 +270,29 @@ sample_rows_kernel(const float *__restrict__ logits, int n, float temp, float to
 // logits [rows, n] -> tokens [rows]; temp <= 0: greedy.  probs: scratch [rows, n] floats.
 // u (device, [rows], nullable) are explicit uniforms in [0, 1); otherwise rng [rows]
 // holds the rows' splitmix64 states and is advanced by one draw.
+template <int CL>
+static int sample_launch(const float *logits, int n, int rows, float temp, float top_p, const double *u, unsigned long long *rng,
+                         float *probs, int32_t *out, cudaStream_t st) {
+    // slices up to 160 KB stay in shared memory (clusters of eight: vocabularies up to 327,680), longer ones in `probs`
+    const size_t slice = (size_t)ceil_div(n, CL) * sizeof(float);
+    const int in_smem = slice <= 160 * 1024;
+    if (in_smem && ensure_dyn_smem((const void *)sample_rows_kernel<CL>, slice)) return 1;
+    launch_k(sample_rows_kernel<CL>, rows * CL, SMP_THREADS, in_smem ? slice : 0, st, logits, n, temp, top_p, u, rng, probs,
+             in_smem, out);
+    APUS_LAUNCHED();
+    return 0;
+}
+
 int sample_rows(const float *logits, int n, int rows, float temp, float top_p, const double *u,
                 unsigned long long *rng, float *probs, int32_t *out, cudaStream_t st) {
     if (rows <= 0) return 0;
     if (temp <= 0.f) return argmax_rows(logits, n, rows, out, st);
     APUS_REQUIRE(u || rng, "sample: neither uniforms nor generator states given");
-    // slices up to 160 KB stay in shared memory (vocabularies up to 327,680), longer ones in `probs`
-    const size_t slice = (size_t)ceil_div(n, SMP_CL) * sizeof(float);
-    const int in_smem = slice <= 160 * 1024;
-    if (in_smem && ensure_dyn_smem((const void *)sample_rows_kernel, slice)) return 1;
-    launch_k(sample_rows_kernel, rows * SMP_CL, SMP_THREADS, in_smem ? slice : 0, st, logits, n, temp, top_p, u, rng, probs,
-             in_smem, out);
-    APUS_LAUNCHED();
-    return 0;
+    // Short rows leave a cluster nothing to share out but its barriers, and fewer clusters than CTAs fit the GPU: one CTA
+    // per row up to 2,048 entries (B200, 256 entries: 1 row 17.6 us with one CTA, 31.0 with eight, 64 rows 18.5 / 154;
+    // 2,000 entries, 1 row 22.4 / 32.2; 8,192 entries 37.8 / 34.0).
+    return n <= 2048 ? sample_launch<1>(logits, n, rows, temp, top_p, u, rng, probs, out, st)
+                     : sample_launch<8>(logits, n, rows, temp, top_p, u, rng, probs, out, st);
 }
 
 }  // namespace apus

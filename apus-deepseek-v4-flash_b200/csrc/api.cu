@@ -347,10 +347,12 @@ int expert_dev(DevQW *w1, DevQW *w2, DevQW *w3, float limit, const float *x, int
     APUS_REQUIRE(w1->fmt == w3->fmt && w1->fmt == w2->fmt && w1->O == w3->O && w1->K == w3->K &&
                  w2->K == w1->O && w2->O == w1->K, "expert: inconsistent weight shapes");
     if (act_quant(x, nullptr, rows, w1->K, ws.xq, ws.xs, nullptr, st)) return 1;
-    if (ws.h2 && w1->tc && w3->tc && wide_rows(rows, w1->K)) {
-        // The paired kernel reads a weight tile once per 32 rows.  From 64 rows on gate and up go through the 128-row
-        // kernel one after the other, and the activation is applied where their product is quantised: the same sums
-        // and roundings.  B200, 2,048 rows: 285 us in pairs, about 190 us so.
+    const long long pair_ctas = (long long)ceil_div(w1->O, 128) * ceil_div(rows, 32);
+    if (ws.h2 && w1->tc && w3->tc && wide_rows(rows, w1->K) && pair_ctas > 148) {
+        // The paired kernel reads a weight tile once per 32 rows.  When its CTAs no longer have an SM each, gate and up go
+        // through the 128-row kernel one after the other, and the activation is applied where their product is
+        // quantised: the same sums and roundings.  B200, whole expert, in pairs / so (4096 x 2048, 16 x rows / 32 CTAs):
+        // 64 rows 59 / 71 us, 257 rows (144 CTAs) 65 / 78, 320 rows (160) 97 / 80, 2,048 rows 371 / 197.
         if (qgemm_dev(w1, nullptr, ws.xq, ws.xs, rows, ws.h, true, 0.f, st) ||
             qgemm_dev(w3, nullptr, ws.xq, ws.xs, rows, ws.h2, true, 0.f, st) ||
             swiglu_quant(ws.h, ws.h2, limit, rows, w1->O, ws.hq, ws.hs, st))

@@ -64,7 +64,7 @@ int ApusCudaMoe::ensure(int s, int n_rout) {
         if (b_logits.get(S * E * 4, nullptr) || b_sp.get(S * E * 4, nullptr) ||
             b_biased.get(S * E * 4, nullptr) || b_idx.get(S * topk * 4, nullptr) ||
             b_wgt.get(S * topk * 4, nullptr) || b_shared.get(S * dim * 4, nullptr) ||
-            b_sh_h.get(2 * S * inter * 4, nullptr) || b_sh_hq.get(S * inter, nullptr) ||
+            b_sh_h.get(S * inter * 4, nullptr) || b_sh_hq.get(S * inter, nullptr) ||
             b_sh_hs.get(S * (inter / 128) * 4, nullptr) || b_ids.get(S * 8, nullptr) ||
             b_sh_xq.get(S * dim, nullptr) || b_sh_xs.get(S * (dim / 128) * 4, nullptr) ||
             b_tab.get(S * topk * 8, nullptr))
@@ -198,9 +198,11 @@ static int experts_run(ApusCudaMoe *m, const float *xrows, int n_rows, const int
 }
 
 static int shared_run(ApusCudaMoe *m, const float *x, int s, float *shared, cudaStream_t st) {
-    // own activation-code buffers: the shared expert may run beside the routed experts
+    // own activation-code buffers: the shared expert may run beside the routed experts.  The up projection of many rows
+    // waits for its activation in the output rows, which the down projection writes last.
+    const bool park = m->dim >= m->inter && ((uintptr_t)shared & 15) == 0;
     ExpertWs ws = {m->b_sh_h.as<float>(), m->b_sh_xq.as<uint8_t>(), m->b_sh_hq.as<uint8_t>(),
-                   m->b_sh_xs.as<float>(), m->b_sh_hs.as<float>(), m->b_sh_h.as<float>() + (size_t)m->cap_s * m->inter};
+                   m->b_sh_xs.as<float>(), m->b_sh_hs.as<float>(), park ? shared : nullptr};
     return expert_dev(&m->sw1, &m->sw2, &m->sw3, m->limit, x, s, shared, ws, st);
 }
 

@@ -102,7 +102,7 @@ int qgemm_dev(DevQW *w, DevQW *other, const uint8_t *acodes, const float *ascale
 // SwiGLU expert on device rows (MXFP4 or FP8 by the handles' fmt).
 struct ExpertWs {
     float *h; uint8_t *xq, *hq; float *xs, *hs;
-    float *h2 = nullptr;      // optional, as large as h: many rows then run gate and up as two 128-row GEMMs
+    float *h2 = nullptr;      // optional, as large as h, may be the output: many rows then run gate and up as two 128-row GEMMs
 };
 int expert_dev(DevQW *w1, DevQW *w2, DevQW *w3, float limit, const float *x, int rows,
                float *out, const ExpertWs &ws, cudaStream_t st);

@@ -467,7 +467,7 @@ int apus_cuda_moe_timing_read(ApusCudaMoe *m, double *ms_gate_up, double *ms_dow
     return 0;
 }
 
-/* Work items (expert x up to 32 rows) launched since the last reset: at decode
+/* Work items (expert x up to 32 rows, 64 for long prompts) launched since the last reset: at decode
  * sizes one per distinct expert touched, i.e. the number of expert weight sets
  * the GEMV kernels streamed. */
 long long apus_cuda_moe_work_items(ApusCudaMoe *m, int reset) {

@@ -504,16 +504,15 @@ sparse_scores_tile_kernel(const float *__restrict__ q, int h, int d, const int32
     const size_t esz = BF16 ? 2 : 4;
     const int nchunk = d / KC;
     // copy u of this thread: row (tid + NT u) / 8, 16-byte segment tid % 8; its rows are the same in every chunk
-    constexpr int NKV = (CANDS * 8 + NT - 1) / NT;
-    static_assert((CANDS * 8 % NT == 0 || NKV == 1) && NT % 8 == 0, "row copies must divide among the threads");
-    const bool copies = tid < CANDS * 8;                        // the smallest tile has fewer copies than threads
+    constexpr int NKV = CANDS * 8 / NT;
+    static_assert(CANDS * 8 % NT == 0 && NT % 8 == 0, "row copies must divide among the threads");
     const char *rowp[NKV];
     const char *dummy = reinterpret_cast<const char *>(kv_a ? kv_a : kv_b);
 #pragma unroll
     for (int u = 0; u < NKV; u++) {
         const int j = j0 + ((tid + NT * u) >> 3);
         const char *ptr = nullptr;
-        if (copies && j < n) {
+        if (j < n) {
             const int32_t id = ids[(size_t)t * idxw + j];
             ptr = id < na ? reinterpret_cast<const char *>(kv_a) + (size_t)own * a_stride + (size_t)id * d * esz
                           : reinterpret_cast<const char *>(kv_b) + (size_t)own * b_stride + (size_t)(id - na) * d * esz;
@@ -524,7 +523,7 @@ sparse_scores_tile_kernel(const float *__restrict__ q, int h, int d, const int32
     auto q_of = [&](int st) { return reinterpret_cast<float *>(ss_raw + (size_t)st * Cf::STAGE); };
     auto kv_of = [&](int st) { return reinterpret_cast<uint32_t *>(ss_raw + (size_t)st * Cf::STAGE) + Cf::Q_WORDS; };
     auto kv_stage = [&](int c) {
-        if (c < nchunk && copies) {
+        if (c < nchunk) {
             uint32_t *dst = kv_of(c % SS_NS);
 #pragma unroll
             for (int u = 0; u < NKV; u++)
@@ -563,7 +562,6 @@ sparse_scores_tile_kernel(const float *__restrict__ q, int h, int d, const int32
     bool kv_bad = false;
     // this thread's own copies of chunk c have landed: are they all in the window?
     auto kv_check = [&](int c) {
-        if (!copies) return;
         const uint32_t *src = kv_of(c % SS_NS);
         uint32_t low = 0, mx = 0, mn = 0xffffffffu;             // f32 rows: low halves, largest and smallest non-zero |v|
 #pragma unroll

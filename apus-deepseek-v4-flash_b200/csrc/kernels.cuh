@@ -63,7 +63,7 @@ int gemm_small(const GemmSmallArgs &a, cudaStream_t st);
 // ---- tcgen05 MXFP4 GEMM on the reference weight storage (gemm_tc.cu) ---------------------
 struct TcGroup {
     int a_row;                // first row of this work item's matrix in the weight slab
-    int row0, nrows;          // activation rows [row0, row0+nrows) in sorted order, nrows <= 32
+    int row0, nrows;          // activation rows [row0, row0+nrows) in sorted order, nrows <= 32 (64: TcArgs::rows64)
     int pad;
 };
 struct TcArgs {

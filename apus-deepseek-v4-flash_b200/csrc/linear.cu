@@ -378,35 +378,35 @@ f32_linear_seq_kernel(const void *__restrict__ wv, const float *__restrict__ x, 
 // and lasts as long as one chain of K adds, four cycles each.  What the kernel above adds to that chain is a
 // CTA-wide barrier per K tile behind a pass of staging threads.  Here a producer thread keeps a ring of K tiles
 // (32 weight rows and the CTA's tokens, four 32-wide TMA boxes each with 128-byte swizzled rows) in flight, and every
-// chain warp (a lane owns one output row x MTT tokens) runs through the ring on its own, waiting for a tile's
+// chain warp (a lane owns one output row, the warp one token) runs through the ring on its own, waiting for a tile's
 // mbarrier and releasing it with one arrival; the operands of a step of eight k are read one step ahead, across tile
 // borders too.  Same products, same order of adds, same bits.
 // One chain per lane walks at 4.14 cycles per k.  (Bulk copies, one per row, were
 // slower than the kernel above: some 33 cycles each whatever their size.)  B200, K = 4096: one token
 // 24.4 -> 19.3 us, two to eight tokens 34 -> 19 us, 32 tokens x 256 rows (the gate) 26.6 -> 17.5 us.
-template <int MTT, int CW, int NST>
+template <int CW, int NST>
 struct ChainCfg {
-    static constexpr int TOK = MTT * CW, XBOX = TOK * 128 < 1024 ? 1024 : TOK * 128;        // bytes of a 32-wide box of x
+    static constexpr int XBOX = CW * 128 < 1024 ? 1024 : CW * 128;       // bytes of a 32-wide box of x: a row per chain warp
     static constexpr int STAGE = 4 * (4096 + XBOX), SMEM = NST * STAGE + 2 * NST * 8 + 1024;
     static_assert(XBOX % 1024 == 0, "a swizzled box starts on 1024 bytes");
 };
-template <int MTT, int CW, int NST>
+template <int CW, int NST>
 __global__ void __launch_bounds__(32 * (CW + 1))
 f32_chain_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
                  const __grid_constant__ CUtensorMap tm_x, float *__restrict__ out, int M, int K, int O, int flags,
                  long long out_stride, int out_ld, int *__restrict__ status) {
     APUS_PDL_WAIT();
     APUS_PDL_GO();
-    using Cf = ChainCfg<MTT, CW, NST>;
-    constexpr int STAGE = Cf::STAGE, XBOX = Cf::XBOX, TOK = Cf::TOK;
+    using Cf = ChainCfg<CW, NST>;
+    constexpr int STAGE = Cf::STAGE, XBOX = Cf::XBOX;
     extern __shared__ unsigned char ch_raw[];
     __shared__ volatile int s_abort;
     unsigned char *smem = reinterpret_cast<unsigned char *>(((uintptr_t)ch_raw + 1023) & ~(uintptr_t)1023);
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + (size_t)NST * STAGE), *empty = full + NST;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int o0 = blockIdx.x * 32, m0 = blockIdx.y * TOK, nt = (K + SQ_KT - 1) / SQ_KT;
+    const int o0 = blockIdx.x * 32, m0 = blockIdx.y * CW, nt = (K + SQ_KT - 1) / SQ_KT;
     out += blockIdx.z * out_stride;
-    const int warps = (min(TOK, M - m0) + MTT - 1) / MTT;                 // chain warps with a token
+    const int warps = min(CW, M - m0);                                    // chain warps with a token
     if (tid == 0) {
         for (int i = 0; i < NST; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], (uint32_t)warps); }
         s_abort = 0;
@@ -421,7 +421,7 @@ f32_chain_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constan
                 const int st = t % NST, k0 = t * SQ_KT, boxes = (min(SQ_KT, K - k0) + 31) / 32;
                 if (!mbar_wait(&empty[st], ((uint32_t)(t / NST) & 1u) ^ 1u, &s_abort)) { fail = 41; break; }
                 unsigned char *dst = smem + (size_t)st * STAGE;
-                mbar_expect_tx(&full[st], (uint32_t)boxes * (4096 + TOK * 128));
+                mbar_expect_tx(&full[st], (uint32_t)boxes * (4096 + CW * 128));
                 for (int b = 0; b < boxes; b++) {
                     tma_load_2d(dst + b * 4096, tm_w, k0 + 32 * b, o0, &full[st]);
                     tma_load_2d(dst + 4 * 4096 + b * XBOX, &tm_x, k0 + 32 * b, m0, &full[st]);
@@ -429,13 +429,11 @@ f32_chain_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constan
             }
         }
     } else if (warp < warps) {
-        float acc[MTT];
-#pragma unroll
-        for (int j = 0; j < MTT; j++) acc[j] = 0.f;
-        struct Ops { float4 wa, wb, xa[MTT], xb[MTT]; } A, B;
+        float acc = 0.f;
+        struct Ops { float4 wa, wb, xa, xb; } A, B;
         // word c of a row sits at chunk c ^ (row % 8): the row's address with its own chunk bits, then xor c
         const uint32_t wrow = smem_u32(smem) + lane * 128 + (lane & 7) * 16;
-        const uint32_t x0 = smem_u32(smem) + 4 * 4096;
+        const uint32_t xrow = smem_u32(smem) + 4 * 4096 + warp * 128 + (warp & 7) * 16;
         auto lds = [](uint32_t addr) {
             float4 v;
             asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
@@ -443,17 +441,11 @@ f32_chain_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constan
         };
         auto load = [&](Ops &o, uint32_t base, int s) {
             const uint32_t c = (uint32_t)(2 * (s & 3)) * 16, w = wrow + base + (uint32_t)(s >> 2) * 4096;
+            const uint32_t x = xrow + base + (uint32_t)(s >> 2) * XBOX;
             o.wa = lds(w ^ c); o.wb = lds(w ^ (c + 16));
-#pragma unroll
-            for (int j = 0; j < MTT; j++) {
-                const uint32_t r = (uint32_t)(warp * MTT + j), x = x0 + base + (uint32_t)(s >> 2) * XBOX + r * 128 + (r & 7) * 16;
-                o.xa[j] = lds(x ^ c); o.xb[j] = lds(x ^ (c + 16));
-            }
+            o.xa = lds(x ^ c); o.xb = lds(x ^ (c + 16));
         };
-        auto walk = [&](const Ops &o) {
-#pragma unroll
-            for (int j = 0; j < MTT; j++) acc[j] = seq_walk8<false>(acc[j], o.wa, o.wb, o.xa[j], o.xb[j]);
-        };
+        auto walk = [&](const Ops &o) { acc = seq_walk8<false>(acc, o.wa, o.wb, o.xa, o.xb); };
         auto wait = [&](int t) {
             if (!__all_sync(0xffffffffu, mbar_wait(&full[t % NST], (uint32_t)(t / NST) & 1u, &s_abort))) fail = 42;
         };
@@ -482,12 +474,7 @@ f32_chain_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constan
             if (!fail)
                 for (int s = 0; s < (K - nfull * SQ_KT) / 8; s++) { load(A, (uint32_t)(nfull % NST) * STAGE, s); walk(A); }
         }
-        if (!fail && o0 + lane < O)
-#pragma unroll
-            for (int j = 0; j < MTT; j++) {
-                const int m = m0 + warp * MTT + j;
-                if (m < M) out[(size_t)m * out_ld + o0 + lane] = (flags & APUS_CUDA_R_OUT) ? bf16_round(acc[j]) : acc[j];
-            }
+        if (!fail && o0 + lane < O) out[(size_t)(m0 + warp) * out_ld + o0 + lane] = (flags & APUS_CUDA_R_OUT) ? bf16_round(acc) : acc;
     }
     if (fail) {
         s_abort = 1;
@@ -508,18 +495,18 @@ static int make_f32_map(void *map, const float *base, long long rows, int K, lon
     APUS_REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled(f32 [%lld,%d]) failed: %d", rows, K, (int)r);
     return 0;
 }
-template <int MTT, int CW, int NST>
+template <int CW, int NST>
 static int chain_launch(const float *w, long long ws, const float *x, int x_ld, float *out, long long os, int out_ld,
                         int batch, int M, int K, int O, int flags, cudaStream_t st) {
-    using Cf = ChainCfg<MTT, CW, NST>;
-    auto kern = f32_chain_kernel<MTT, CW, NST>;
+    using Cf = ChainCfg<CW, NST>;
+    auto kern = f32_chain_kernel<CW, NST>;
     int *status = wait_word();
     if (!status || ensure_dyn_smem((const void *)kern, Cf::SMEM + 16)) return 1;
     alignas(64) unsigned char m0[128], m1[128], mx[128];
     if (make_f32_map(m0, w, O, K, K, 32) || make_f32_map(m1, w + (batch > 1 ? ws : 0), O, K, K, 32) ||
-        make_f32_map(mx, x, M, K, x_ld, Cf::TOK))
+        make_f32_map(mx, x, M, K, x_ld, CW))
         return 1;
-    const dim3 grid((unsigned)ceil_div(O, 32), (unsigned)ceil_div(M, Cf::TOK), (unsigned)batch);
+    const dim3 grid((unsigned)ceil_div(O, 32), (unsigned)ceil_div(M, CW), (unsigned)batch);
     launch_k(kern, grid, 32 * (CW + 1), Cf::SMEM, st, *reinterpret_cast<const CUtensorMap *>(m0),
              *reinterpret_cast<const CUtensorMap *>(m1), *reinterpret_cast<const CUtensorMap *>(mx), out, M, K, O, flags, os, out_ld, status);
     return 0;
@@ -561,12 +548,14 @@ static int launch_linear_seq(const void *w, long long ws, const float *x, long l
                           (batch == 1 || (batch == 2 && xs == 0)) && !(flags & APUS_CUDA_R_IN);
 #define CHAIN_ARGS (const float *)w, ws, x, x_ld, out, os, out_ld, batch, M, K, O, flags, st
         if (maps) {
-            // Up to two CTAs per SM one chain per lane, the fastest walk.  With more, every warp's reads of the weight
+            // One token always, two per CTA up to two CTAs per SM.  With more of those, every warp's reads of the weight
             // tile fill the shared-memory pipe (32 tokens per CTA, four per lane: 85 us where the kernel above takes 43).
+            // K = 4096, kernel above / this one: 1 token x 256 rows 22.3 / 15.9 us, x 9,504 (297 CTAs, one per SM at a
+            // time) 65 / 47, x 129,280 595 / 433; 2 tokens x 9,472 rows (296 CTAs) 53.5 / 26.6, 8 x 2,368 31.8 / 22.4.
             const long long ctas2 = (long long)ceil_div(O, 32) * batch * ceil_div(M, 2);
-            if (M == 1) return chain_launch<1, 1, 6>(CHAIN_ARGS);
-            if (ctas2 <= 148) return chain_launch<1, 2, 6>(CHAIN_ARGS);
-            if (ctas2 <= 296) return chain_launch<1, 2, 4>(CHAIN_ARGS);
+            if (M == 1) return chain_launch<1, 6>(CHAIN_ARGS);
+            if (ctas2 <= 148) return chain_launch<2, 6>(CHAIN_ARGS);
+            if (ctas2 <= 296) return chain_launch<2, 4>(CHAIN_ARGS);
         }
 #undef CHAIN_ARGS
     }

@@ -17,9 +17,10 @@
 // atomic adds (the reference's double sums differ from exact sums by ~1e-16,
 // which can only matter for a u within that distance of a boundary).
 //
-// A row is spread over a cluster of eight CTAs whose slices of the probabilities
-// stay in their shared memory for all sweeps (max, exponentials, eight
-// histogram passes).  What bounds it is latency: eleven cluster barriers and
+// A row of more than 2,048 entries is spread over a cluster of eight CTAs whose
+// slices of the probabilities stay in their shared memory for all sweeps (max,
+// exponentials, eight histogram passes).  What bounds it is latency: twelve
+// cluster barriers (one more when the uniform comes from the generator) and
 // the sweeps between them; the row itself is read once.  Vocabulary 129,280,
 // five rows: about 4,000 us with one CTA per row sweeping L2 and adding 64-bit
 // masses to shared memory (a compare-and-swap loop per add, all lanes on the

@@ -385,8 +385,9 @@ gemm_tc8_wide_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
                     as[j] = __fmul_rn(as[j], ws);
-                    const bool pow2 = (__float_as_uint(as[j]) & 0x7fffffu) == 0u;
-                    ok = ok && (as[j] == 0.f || (pow2 && as[j] >= 7.88860905e-31f && as[j] <= 1.23794004e27f));     // 2^-100, 2^90
+                    // the bits turned left by nine: the exponent alone (27 for 2^-100 .. 217 for 2^90) of a positive power of two
+                    const uint32_t u = __float_as_uint(as[j]);
+                    ok = ok && (u == 0u || __funnelshift_l(u, u, 9) - 27u <= 190u);
                 }
                 *reinterpret_cast<float4 *>(s_sw + b * T8W_N + 4 * lane) = make_float4(as[0], as[1], as[2], as[3]);
                 const int all = __all_sync(0xffffffffu, ok);
